@@ -28,7 +28,10 @@ namespace rd {
 namespace {
 
 struct FastOptics {
-  float cxh, cxl, cyh, cyl, uh, ul;  // f64 constants split into FP32 pairs
+  float uh, ul;   // f64 unscale split into an FP32 pair
+  float2 oh, ol;  // centre * unscale (x, y) split alike
+  float2 err;     // what x and y may be off by before they are rounded
+  float neg_zero;
 };
 
 struct OpticsParams {
@@ -41,6 +44,7 @@ struct OpticsParams {
   double cx, cy, unscale;
   int dist_model;
   float d0, d1, d2;
+  float inv_k1;      // Poly3: 1 / d0
   int tca_model;
   float tr[3], tb[3];
   unsigned* error;
@@ -117,16 +121,36 @@ __device__ __forceinline__ float df_round(df v, bool& amb) {
   return r;
 }
 
-// (n + c) * unscale in f64, narrowed to f32 (plan.rs:476-478).
-__device__ __forceinline__ float post_transform(float n, float ch, float cl, const FastOptics& f, double c64,
-                                                double unscale, bool& fell_back) {
-  df t = two_sum(n, ch);
-  t = fast_two_sum(t.h, t.l + cl);
-  bool amb = false;
-  const float r = df_round(df_mul(t, {f.uh, f.ul}), amb);
-  if (!amb) return r;
-  fell_back = true;
-  return (float)(((double)n + c64) * unscale);
+// ---- packed FP32: x and y of a coordinate, or two taps, in one instruction ----
+// Products are fused multiply-adds with -0.0 (`z`, from a launch argument):
+// the exact product rounded once, and nothing for the compiler to contract.
+__device__ __forceinline__ float2 pmul(float2 a, float2 b, float2 z) { return __ffma2_rn(a, b, z); }
+__device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 pneg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 pair(float v) { return make_float2(v, v); }
+
+// (n + c) * unscale in f64, narrowed to f32 (plan.rs:476-478), of x and y, as
+// n * unscale + (c * unscale) in double-float: the two differ by a few 2^-53 of
+// the coordinate, the double-float sum by a few 2^-46. The sum is rounded with
+// the error bound `err` (2^-40 of the largest coordinate) added and taken away
+// (Ziv's test): when both give the same f32, so does the f64 value; otherwise
+// `sure` is cleared and the caller takes the f64 form. 15 packed instructions
+// against about 90 of the double-float form of the expression as it stands
+// (two normalised double-float operations and an exponent test, for x and y).
+__device__ __forceinline__ float2 post_transform(float2 n, const FastOptics& f, float2 z, bool& sure) {
+  const float2 uh = pair(f.uh);
+  const float2 ph = pmul(n, uh, z);
+  const float2 pl = __ffma2_rn(n, uh, pneg(ph));
+  const float2 sum = padd(ph, f.oh);
+  const float2 bb = padd(sum, pneg(ph));
+  const float2 sl = padd(padd(ph, pneg(padd(sum, pneg(bb)))), padd(f.oh, pneg(bb)));
+  const float2 low = padd(sl, padd(pl, __ffma2_rn(n, pair(f.ul), f.ol)));
+  const float2 r = padd(sum, padd(low, f.err)), r2 = padd(sum, padd(low, pneg(f.err)));
+  sure = sure && r.x == r2.x && r.y == r2.y;
+  return r;
+}
+__device__ __forceinline__ float post_transform_f64(float n, double c, double unscale) {
+  return (float)(((double)n + c) * unscale);
 }
 
 // Poly5 inverse from f32 (x, y): the f64 Newton result, computed through the
@@ -178,105 +202,312 @@ __device__ __forceinline__ void undistort_poly5_fast(float x, float y, float a, 
   oy = ry;
 }
 
-// cubic_weight (resample.rs) at the four distances x - (fx - 1) .. x - (fx + 2)
-// of a footprint with fx = floor(x) >= 1. Those differences are exact and lie
-// in [1, 2), [0, 1), [-1, 0) and [-2, -1), so each weight takes one fixed
-// branch: |d| <= 1 for the middle two, 1 < |d| < 2 for the outer two. The
-// outer distances reach 1 or 2 only when x is an integer, where the
-// reference's branch and this one both give +0.0.
-__device__ __forceinline__ void cubic_weights(float x, int fx, float (&w)[4]) {
-  const float a0 = fabsf(x - (float)(fx - 1));
-  const float a1 = fabsf(x - (float)fx);
-  const float a2 = fabsf(x - (float)(fx + 1));
-  const float a3 = fabsf(x - (float)(fx + 2));
-  w[0] = -0.5f * a0 * a0 * a0 + 2.5f * a0 * a0 - 4.0f * a0 + 2.0f;
-  w[1] = 1.5f * a1 * a1 * a1 - 2.5f * a1 * a1 + 1.0f;
-  w[2] = 1.5f * a2 * a2 * a2 - 2.5f * a2 * a2 + 1.0f;
-  w[3] = -0.5f * a3 * a3 * a3 + 2.5f * a3 * a3 - 4.0f * a3 + 2.0f;
+// Poly3 inverse from f32 (x, y), as above: with R = f32(rd / k1) and e =
+// rd / k1 - R, F(rd) = rd^3 + e, so a break at step 0 gives ratio 1 and one at
+// step 1 gives ratio = 1 - (u + e / rd) / (3 u + 1 / k1) for u = rd^2. In
+// double-float R and e are the two halves of the product rd / k1. A Poly3 lens
+// has no radial table (its freeze is ambiguous), so every pixel comes here; the
+// f64 iteration took 4.32 ms per 8256x5504 frame at the FP64 rate.
+__device__ __forceinline__ void undistort_poly3_fast(float x, float y, float inv_k1, float& ox, float& oy,
+                                                     bool& need_more) {
+  ox = x;
+  oy = y;
+  const float s = x * x + y * y;
+  if (s == 0.0f) return;
+  const float rh = sqrtf(s);
+  const float rl = __fmaf_rn(-rh, rh, s) * __fdividef(0.5f, rh);  // sqrt(s) = rh + rl
+  df p = two_prod(rh, inv_k1);
+  p = fast_two_sum(p.h, p.l + rl * inv_k1);
+  const float thr = 1.0e-5f;
+  const float f0 = s * rh + p.l;
+  const float d0 = 3.0f * s + inv_k1;
+  const float step = __fdividef(f0, d0);
+  const float f1 = 3.0f * rh * step * step;  // F(ru1) = 3 rd step^2 - step^3
+  // p.h is R unless p.l is within 2^-18 of half its ulp. 1 / k1 below 3e4 keeps e below 1e-3, so that f0 is good to
+  // 1e-10 (and to 2^-23 of itself) and the f64 iteration's own rounding is far below the margins of the tests.
+  const bool plain = s > 1.0e-12f && s < 1.0e2f && fabsf(inv_k1) > 1.0e-2f && fabsf(inv_k1) < 3.0e4f &&
+                     fabsf(d0) > 0.25f * fabsf(inv_k1) && p.h + p.l * 1.0000038f == p.h;
+  if (!plain) {
+    need_more = true;
+    return;
+  }
+  if (fabsf(f0) < thr * (1.0f - 1.0e-4f)) return;  // frozen at the input
+  if (fabsf(f0) <= thr * (1.0f + 1.0e-4f) || !(fabsf(f1) < thr * 0.9f)) {
+    need_more = true;
+    return;
+  }
+  const df d = df_add(two_prod(s, 3.0f), {inv_k1, 0.0f});
+  const df q = df_div(two_sum(s, __fdividef(p.l, rh)), d);
+  const df ratio = fast_two_sum(1.0f, -q.h);
+  const df rr = {ratio.h, ratio.l - q.l};
+  bool amb = !(rr.h > 0.0f);
+  const float rx = df_round(df_mul_f(rr, x), amb);
+  const float ry = df_round(df_mul_f(rr, y), amb);
+  if (amb) {
+    need_more = true;
+    return;
+  }
+  ox = rx;
+  oy = ry;
 }
 
-// resample.rs:3-41. Returns false for a non-finite coordinate or a footprint
-// that leaves the image.
+// The Newton inversion of lens_undistort and lens_tca_poly3 step by step in
+// double-float, for what the closed forms do not cover: each iterate is within
+// a few 2^-45 of the f64 one. False where a break test or a rounding is too
+// close to call; the caller then takes the f64 iteration. `model` as
+// lens_undistort's, 4 for the TCA polynomial (k0, k1, k2 = v, c, b).
+__device__ __forceinline__ df df_sub(df x, df y) { return df_add(x, {-y.h, -y.l}); }
+__device__ bool newton_df(int model, float k0, float k1, float k2, float x, float y, float& ox, float& oy) {
+  const float s = x * x + y * y;
+  if (!(s > 1.0e-12f && s < 1.0e4f)) return false;
+  const float rh = sqrtf(s);
+  const df rd = fast_two_sum(rh, __fdividef(__fmaf_rn(-rh, rh, s), 2.0f * rh));
+  df target = rd;
+  float inv_k1 = 0.0f;
+  if (model == 1) {
+    inv_k1 = 1.0f / k0;
+    if (!(fabsf(inv_k1) > 1.0e-4f && fabsf(inv_k1) < 1.0e8f)) return false;
+    const df p = df_mul_f(rd, inv_k1);
+    bool amb = false;
+    target = {df_round(p, amb), 0.0f};
+    if (amb) return false;
+  }
+  df ru = rd;
+  for (int k = 0; k < 7; ++k) {
+    const df r2 = df_mul(ru, ru);
+    df f, d;
+    float size;  // the magnitude that the rounding errors of f go with
+    if (model == 1) {
+      f = df_sub(df_add(df_mul(r2, ru), df_mul_f(ru, inv_k1)), target);
+      d = df_add(df_mul_f(r2, 3.0f), {inv_k1, 0.0f});
+      size = fabsf(r2.h * ru.h) + fabsf(target.h);
+    } else if (model == 2) {
+      const df r4 = df_mul(r2, r2), ar = df_mul_f(r2, k0), br = df_mul_f(r4, k1);
+      f = df_sub(df_mul(ru, df_add({1.0f, 0.0f}, df_add(ar, br))), target);
+      d = df_add({1.0f, 0.0f}, df_add(df_mul_f(ar, 3.0f), df_mul_f(br, 5.0f)));
+      size = fabsf(ru.h) * (1.0f + fabsf(ar.h) + fabsf(br.h)) + rh;
+    } else if (model == 3) {
+      const df ar = df_mul_f(df_mul(r2, ru), k0), br = df_mul_f(r2, k1), cr = df_mul_f(ru, k2);
+      f = df_sub(df_mul(ru, df_add(df_add(df_add(ar, br), cr), {1.0f, 0.0f})), target);
+      d = df_add(df_add(df_add(df_mul_f(ar, 4.0f), df_mul_f(br, 3.0f)), df_mul_f(cr, 2.0f)), {1.0f, 0.0f});
+      size = fabsf(ru.h) * (1.0f + fabsf(ar.h) + fabsf(br.h) + fabsf(cr.h)) + rh;
+    } else {
+      const df br = df_mul_f(r2, k2), cr = df_mul_f(ru, k1);
+      f = df_sub(df_mul(ru, df_add(df_add(br, cr), {k0, 0.0f})), target);
+      d = df_add(df_add(df_mul_f(br, 3.0f), df_mul_f(cr, 2.0f)), {k0, 0.0f});
+      size = fabsf(ru.h) * (fabsf(k0) + fabsf(br.h) + fabsf(cr.h)) + rh;
+    }
+    const float margin = 1.0e-5f * 1.0e-6f + size * 1.8189894e-12f;  // 2^-39 of the terms
+    if (!(fabsf(f.h) < 1.0e30f) || !(fabsf(d.h) > 1.0e-3f * (model == 1 ? fabsf(inv_k1) : 1.0f))) return false;
+    if (fabsf(fabsf(f.h) - 1.0e-5f) <= margin) return false;
+    if (fabsf(f.h) < 1.0e-5f) {
+      if (!(ru.h > 0.0f)) return false;
+      if (k == 0) {  // ru / rd is 1 exactly
+        ox = x;
+        oy = y;
+        return true;
+      }
+      const df ratio = df_div(ru, rd);
+      bool amb = false;
+      ox = df_round(df_mul_f(ratio, x), amb);
+      oy = df_round(df_mul_f(ratio, y), amb);
+      return !amb;
+    }
+    ru = df_sub(ru, df_div(f, d));
+    if (!(ru.h > 1.0e-3f * rh && ru.h < 1.0e3f * rh)) return false;
+  }
+  return false;
+}
+
+// cubic_weight (resample.rs) at the four distances x - (fx - 1) .. x - (fx + 2)
+// of a footprint with fx = floor(x) >= 1, from d = x - fx. Those differences
+// are exact and lie in [1, 2), [0, 1), [-1, 0) and [-2, -1), so they are d + 1,
+// d, d - 1 and d - 2, and each weight takes one fixed branch: |d| <= 1 for the
+// middle two, 1 < |d| < 2 for the outer two. The outer distances reach 1 or 2
+// only when x is an integer, where the reference's branch and this one both
+// give +0.0.
+// Of x and y at once. A product with a power of two is exact, so fusing it with
+// the addition that follows changes nothing (0.5 a a a = 0.5 (a a a), 4 a).
+__device__ __forceinline__ void cubic_weights(float2 d, float2 (&w)[4], float2 z) {
+  const float2 one = pair(1.0f), two = pair(2.0f);
+  const float2 a0 = padd(d, one), a2 = padd(one, pneg(d)), a3 = padd(two, pneg(d));
+  auto outer = [&](float2 a) {
+    const float2 cube = pmul(pmul(a, a, z), a, z), square = pmul(pmul(pair(2.5f), a, z), a, z);
+    return padd(__ffma2_rn(pair(-4.0f), a, __ffma2_rn(pair(-0.5f), cube, square)), two);
+  };
+  auto inner = [&](float2 a) {
+    const float2 cube = pmul(pmul(pmul(pair(1.5f), a, z), a, z), a, z), square = pmul(pmul(pair(-2.5f), a, z), a, z);
+    return padd(padd(cube, square), one);
+  };
+  w[0] = outer(a0);
+  w[1] = inner(d);
+  w[2] = inner(a2);
+  w[3] = outer(a3);
+}
+
+// Four samples of a row (the vignetted source values).
 template <bool VIG>
-__device__ __forceinline__ bool cubic_sample(const float* __restrict__ plane, const float* __restrict__ mult, int W,
-                                             int H, float x, float y, float& out) {
-  if (!isfinite(x) || !isfinite(y)) return false;
-  const int fx = (int)floorf(x), fy = (int)floorf(y);
-  if (fx - 1 < 0 || fy - 1 < 0 || fx + 2 >= W || fy + 2 >= H) return false;
+__device__ __forceinline__ void load_taps(const float* __restrict__ plane, const float* __restrict__ mult, long long at,
+                                          float2 (&s)[2], float2 z) {
+  const float* row = plane + at;
+  s[0] = make_float2(__ldg(row), __ldg(row + 1));
+  s[1] = make_float2(__ldg(row + 2), __ldg(row + 3));
+  if (VIG) {
+    const float* mrow = mult + at;
+    s[0] = pmul(s[0], make_float2(__ldg(mrow), __ldg(mrow + 1)), z);
+    s[1] = pmul(s[1], make_float2(__ldg(mrow + 2), __ldg(mrow + 3)), z);
+  }
+}
+// The sum over a footprint (resample.rs:3-41) whose rows are s[0] .. s[3].
+__device__ __forceinline__ float sum_taps(const float2 (*s)[2], float2 d, float2 z) {
+  float2 w[4];
+  cubic_weights(d, w, z);
+  const float2 wx01 = make_float2(w[0].x, w[1].x), wx23 = make_float2(w[2].x, w[3].x);
   float value = 0.0f;
-  float wx[4], wys[4];
-  cubic_weights(x, fx, wx);  // same for every row
-  cubic_weights(y, fy, wys);
 #pragma unroll
-  for (int oy = -1; oy <= 2; ++oy) {
-    const float wy = wys[oy + 1];
-    const float* row = plane + (long long)(fy + oy) * W;
-    const float* mrow = VIG ? mult + (long long)(fy + oy) * W : nullptr;
+  for (int oy = 0; oy < 4; ++oy) {
+    const float2 wy = pair(w[oy].y);
+    const float2 t01 = pmul(s[oy][0], pmul(wy, wx01, z), z), t23 = pmul(s[oy][1], pmul(wy, wx23, z), z);
+    value += t01.x;
+    value += t01.y;
+    value += t23.x;
+    value += t23.y;
+  }
+  return value;
+}
+
+// Output pixels (x, y) and (x, y + 1) from the positions n of their channels
+// (lens units): post-transform, then the Catmull-Rom gather. The footprints of
+// two pixels one above the other mostly lie one row apart, so the second takes
+// three of its rows from the first (62 % of the loads and vignetting products)
+// and loads them again only where the distortion moves it by another column or
+// row. What bounds the gather is the FP32 pipe (about 540 of 640 issue slots a
+// pixel) and the latency of its loads: 0.54 ms per 24 MP frame with the radial
+// table (0.71 with a pixel per thread, scalar weights and the coordinates'
+// double-float form), 1.21 ms per 45 MP frame through a Poly3 lens (4.32 with
+// its Newton steps in f64). A non-finite coordinate or a footprint that leaves the image is an error.
+template <bool VIG>
+__device__ __forceinline__ void gather_pair(const OpticsParams& p, const float (&n0)[6], const float (&n1)[6],
+                                            bool bad0, bool bad1, int x, int y) {
+  const long long plane = (long long)p.W * p.H;
+  const long long o = (long long)y * p.W + x;
+  const bool two = y + 1 < p.H;
+  const float2 z = pair(p.fast.neg_zero);
+  float2 c[6];
+  bool sure = true;
 #pragma unroll
-    for (int ox = -1; ox <= 2; ++ox) {
-      const float weight = wy * wx[ox + 1];
-      float sample = __ldg(row + fx + ox);
-      if (VIG) sample = sample * __ldg(mrow + fx + ox);  // the vignetted source value
-      value += sample * weight;
+  for (int k = 0; k < 3; ++k) {
+    c[k] = post_transform(make_float2(n0[2 * k], n0[2 * k + 1]), p.fast, z, sure);
+    c[3 + k] = post_transform(make_float2(n1[2 * k], n1[2 * k + 1]), p.fast, z, sure);
+  }
+  if (!sure) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      c[k].x = post_transform_f64(n0[2 * k], p.cx, p.unscale);
+      c[k].y = post_transform_f64(n0[2 * k + 1], p.cy, p.unscale);
+      c[3 + k].x = post_transform_f64(n1[2 * k], p.cx, p.unscale);
+      c[3 + k].y = post_transform_f64(n1[2 * k + 1], p.cy, p.unscale);
     }
   }
-  if (!isfinite(value)) return false;
-  out = value;
-  return true;
+  bool bad = bad0 || (two && bad1);
+  const int W = p.W;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float* src = p.in + k * plane;
+    // The conversion saturates and takes NaN to 0, which is outside.
+    const int fx = __float2int_rd(c[k].x), fy = __float2int_rd(c[k].y);
+    const int gx = __float2int_rd(c[3 + k].x), gy = __float2int_rd(c[3 + k].y);
+    const bool in0 = !bad0 && fx >= 1 && fy >= 1 && fx < W - 2 && fy < p.H - 2;
+    const bool in1 = !bad1 && gx >= 1 && gy >= 1 && gx < W - 2 && gy < p.H - 2;
+    float2 s[5][2];
+    float v0 = 0.0f, v1 = 0.0f;
+    if (in0) {
+      const long long at = (long long)(fy - 1) * W + (fx - 1);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) load_taps<VIG>(src, p.mult, at + (long long)r * W, s[r], z);
+      v0 = sum_taps(s, padd(c[k], make_float2(-(float)fx, -(float)fy)), z);
+    }
+    if (two && in1) {
+      const long long at = (long long)(gy - 1) * W + (gx - 1);
+      if (!(in0 && gx == fx && gy == fy + 1)) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) load_taps<VIG>(src, p.mult, at + (long long)r * W, s[1 + r], z);
+      }
+      load_taps<VIG>(src, p.mult, at + 3ll * W, s[4], z);
+      v1 = sum_taps(s + 1, padd(c[3 + k], make_float2(-(float)gx, -(float)gy)), z);
+    }
+    bad = bad || !in0 || (two && !in1) || !isfinite(v0) || !isfinite(v1);
+    p.out[k * plane + o] = isfinite(v0) ? v0 : 0.0f;
+    if (two) p.out[k * plane + o + W] = isfinite(v1) ? v1 : 0.0f;
+  }
+  if (bad) atomicOr(p.error, 8u);
 }
 
-template <bool VIG>
-__global__ void __launch_bounds__(512) optics_kernel(const OpticsParams p) {
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int y = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (x >= p.W || y >= p.H) return;
+// The position of each channel before the post-transform by the Newton path;
+// false when it is not finite. One copy for a thread's two pixels (inlined
+// twice, the code of all models measured 1 % slower).
+__device__ __noinline__ bool newton_positions(const OpticsParams& p, float ix, float iy, float (&n)[6]) {
   float gx, gy;
-  const float ix = p.ix[x], iy = p.iy[y];
-  if (p.dist_model == RD_DISTORTION_POLY5) {
-    bool need_f64 = false;
-    undistort_poly5_fast(ix, iy, p.d0, p.d1, gx, gy, need_f64);
-    if (need_f64) undistort(p, ix, iy, gx, gy);
+  if (p.dist_model == RD_DISTORTION_NONE) {
+    gx = ix;
+    gy = iy;
   } else {
-    undistort(p, ix, iy, gx, gy);
+    bool need_more = true;
+    if (p.dist_model == RD_DISTORTION_POLY5) {
+      need_more = false;
+      undistort_poly5_fast(ix, iy, p.d0, p.d1, gx, gy, need_more);
+    } else if (p.dist_model == RD_DISTORTION_POLY3) {
+      need_more = false;
+      undistort_poly3_fast(ix, iy, p.inv_k1, gx, gy, need_more);
+    }
+    if (need_more && !newton_df(p.dist_model, p.d0, p.d1, p.d2, ix, iy, gx, gy)) undistort(p, ix, iy, gx, gy);
   }
-  bool bad = !isfinite(gx) || !isfinite(gy);
-  float n[6] = {gx, gy, gx, gy, gx, gy};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    n[2 * k] = gx;
+    n[2 * k + 1] = gy;
+  }
   if (p.tca_model == RD_TCA_LINEAR) {
     n[0] = gx * p.tr[0];
     n[1] = gy * p.tr[0];
     n[4] = gx * p.tb[0];
     n[5] = gy * p.tb[0];
   } else if (p.tca_model == RD_TCA_POLY3) {
-    tca_poly3(p.tr, gx, gy, n[0], n[1]);
-    tca_poly3(p.tb, gx, gy, n[4], n[5]);
+    if (!newton_df(4, p.tr[0], p.tr[1], p.tr[2], gx, gy, n[0], n[1])) tca_poly3(p.tr, gx, gy, n[0], n[1]);
+    if (!newton_df(4, p.tb[0], p.tb[1], p.tb[2], gx, gy, n[4], n[5])) tca_poly3(p.tb, gx, gy, n[4], n[5]);
   }
-  const long long plane = (long long)p.W * p.H;
-  const long long o = (long long)y * p.W + x;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    bool fell_back = false;
-    const float sx = post_transform(n[2 * c], p.fast.cxh, p.fast.cxl, p.fast, p.cx, p.unscale, fell_back);
-    const float sy = post_transform(n[2 * c + 1], p.fast.cyh, p.fast.cyl, p.fast, p.cy, p.unscale, fell_back);
-    float v = 0.0f;
-    if (!bad && !cubic_sample<VIG>(p.in + c * plane, p.mult, p.W, p.H, sx, sy, v)) bad = true;
-    p.out[c * plane + o] = v;
-  }
-  if (bad) atomicOr(p.error, 8u);
+  return isfinite(gx) && isfinite(gy);
+}
+
+template <bool VIG>
+__global__ void __launch_bounds__(256, 4) optics_kernel(const OpticsParams p) {
+  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int y = 2 * (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  if (x >= p.W || y >= p.H) return;
+  const float ix = p.ix[x];
+  float n0[6], n1[6];
+  const bool bad0 = !newton_positions(p, ix, p.iy[y], n0);
+  const bool bad1 = !newton_positions(p, ix, p.iy[min(y + 1, p.H - 1)], n1);
+  gather_pair<VIG>(p, n0, n1, bad0, bad1, x, y);
 }
 
 // f32 hypot as the reference gets it (f32::hypot, glibc hypotf): the double
 // sum of the two exact double squares, its double square root, narrowed once.
-// Here the square root is taken in double-float from the exact FP32-pair sum
-// of squares (one Newton correction of sqrtf); the rare result too close to
-// an f32 rounding boundary (or zero, tiny, huge) is recomputed in f64.
+// Here the square root is taken in double-float from the FP32-pair sum of
+// squares (one Newton correction of an approximate root) and rounded by Ziv's
+// test as in post_transform (the root is within a few 2^-45 of the f64 one);
+// the rare result too close to an f32 rounding boundary, and sums outside the
+// plain range, are computed in f64.
 __device__ __forceinline__ float hypot_f32(float x, float y) {
-  const df s = df_add(two_prod(x, x), two_prod(y, y));
-  const float r0 = sqrtf(s.h);
-  const df r2 = two_prod(r0, r0);
-  const float residual = ((s.h - r2.h) - r2.l) + s.l;  // s.h - r2.h is exact
-  bool amb = false;
-  const float r = df_round(fast_two_sum(r0, __fdividef(residual, 2.0f * r0)), amb);
-  if (!amb) return r;
+  const df xx = two_prod(x, x), yy = two_prod(y, y);
+  const df s = two_sum(xx.h, yy.h);
+  const float low = s.l + (xx.l + yy.l);
+  const float inv = rsqrtf(s.h);
+  const float r0 = s.h * inv;
+  const float correction = (__fmaf_rn(-r0, r0, s.h) + low) * (0.5f * inv);
+  const float err = r0 * 9.094947e-13f;  // 2^-40
+  const float r = r0 + (correction + err);
+  if (r == r0 + (correction - err) && s.h > 1.0e-20f && s.h < 1.0e20f) return r;
   return (float)sqrt((double)x * (double)x + (double)y * (double)y);
 }
 
@@ -306,13 +537,8 @@ __global__ void hypot_check_kernel(unsigned first, unsigned last, unsigned long 
 // then plan.rs:136-141's post-transform and the Catmull-Rom gather per
 // channel. `knots` holds [m_r, m_g, m_b, pin] per knot; it is 16 KB and stays
 // in L1.
-template <bool VIG>
-__global__ void __launch_bounds__(512) optics_lut_kernel(const OpticsParams p, const float4* __restrict__ knots,
-                                                         float step) {
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int y = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (x >= p.W || y >= p.H) return;
-  const float ix = p.ix[x], iy = p.iy[y];
+__device__ __forceinline__ void table_positions(const float4* __restrict__ knots, float step, float ix, float iy,
+                                                float (&n)[6]) {
   const float radius = hypot_f32(ix, iy);
   const float position = radius / step;
   const int index = position < (float)(RADIAL_KNOTS - 2) ? (int)position : RADIAL_KNOTS - 2;
@@ -330,19 +556,24 @@ __global__ void __launch_bounds__(512) optics_lut_kernel(const OpticsParams p, c
     m[1] = lo.y * (1.0f - blend) + hi.y * blend;
     m[2] = lo.z * (1.0f - blend) + hi.z * blend;
   }
-  const long long plane = (long long)p.W * p.H;
-  const long long o = (long long)y * p.W + x;
-  bool bad = false;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    bool fell_back = false;
-    const float sx = post_transform(ix * m[c], p.fast.cxh, p.fast.cxl, p.fast, p.cx, p.unscale, fell_back);
-    const float sy = post_transform(iy * m[c], p.fast.cyh, p.fast.cyl, p.fast, p.cy, p.unscale, fell_back);
-    float v = 0.0f;
-    if (!bad && !cubic_sample<VIG>(p.in + c * plane, p.mult, p.W, p.H, sx, sy, v)) bad = true;
-    p.out[c * plane + o] = v;
+  for (int k = 0; k < 3; ++k) {
+    n[2 * k] = ix * m[k];
+    n[2 * k + 1] = iy * m[k];
   }
-  if (bad) atomicOr(p.error, 8u);
+}
+
+template <bool VIG>
+__global__ void __launch_bounds__(256, 4) optics_lut_kernel(const OpticsParams p, const float4* __restrict__ knots,
+                                                         float step) {
+  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int y = 2 * (blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5));
+  if (x >= p.W || y >= p.H) return;
+  const float ix = p.ix[x];
+  float n0[6], n1[6];
+  table_positions(knots, step, ix, p.iy[y], n0);
+  table_positions(knots, step, ix, p.iy[min(y + 1, p.H - 1)], n1);
+  gather_pair<VIG>(p, n0, n1, false, false, x, y);
 }
 
 // Horizontal area pass: one thread per (row, target column, channel-plane).
@@ -532,16 +763,24 @@ Status run_optics_gather(Context& ctx, const rd_optics_desc& o, const float* rgb
     h = (float)v;
     l = (float)(v - (double)h);
   };
-  split(o.center_x, p.fast.cxh, p.fast.cxl);
-  split(o.center_y, p.fast.cyh, p.fast.cyl);
   split(o.norm_unscale, p.fast.uh, p.fast.ul);
-  // Tiles of 32 columns and `rows` rows (one warp per row), tuned across
-  // calls per image shape: the tile only decides which CTA takes which pixel.
+  split(o.center_x * o.norm_unscale, p.fast.oh.x, p.fast.ol.x);
+  split(o.center_y * o.norm_unscale, p.fast.oh.y, p.fast.ol.y);
+  // Coordinates that matter lie within twice the image and the centre; one further out fails its footprint test
+  // in either form.
+  p.fast.err.x = (float)((2.0 * W + std::fabs(o.center_x * o.norm_unscale)) * 0x1p-40);
+  p.fast.err.y = (float)((2.0 * H + std::fabs(o.center_y * o.norm_unscale)) * 0x1p-40);
+  p.fast.neg_zero = -0.0f;
+  p.inv_k1 = 1.0f / o.distortion[0];
+  // Tiles of 32 columns and `rows` rows (one warp per two rows), tuned across
+  // calls per image shape: the tile only decides which CTA takes which pixels.
+  // 32 rows, a CTA of 16 warps, would not hold four CTAs' worth of warps at 64
+  // registers; with fewer registers (54, 48, 40) the gather is 5 to 8 % slower.
   const ShapeKey key{TUNE_OPTICS, W, H, 0};
-  const ShapePick pick = shape_begin(ctx, key, 8, {4, 16});
+  const ShapePick pick = shape_begin(ctx, key, 16, {8});
   const int rows = pick.value;
   const dim3 grid((W + 31) / 32, (H + rows - 1) / rows);
-  const unsigned block = 32u * (unsigned)rows;
+  const unsigned block = 16u * (unsigned)rows;
   const float4* knots = reinterpret_cast<const float4*>(dbuf);
   if (lut && p.mult) {
     RD_LAUNCH(ctx, K_OPTICS, optics_lut_kernel<true><<<grid, block, 0, ctx.stream>>>(p, knots, radial.step));
