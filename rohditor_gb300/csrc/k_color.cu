@@ -41,7 +41,8 @@ struct ColorParams {
 
 // The adjustment chain, output transform, sRGB8 quantisation and histogram
 // bins of one base pixel (index i of a plane of `plane` pixels).
-__device__ __forceinline__ void color_pixel(const ColorParams& p, long long i, long long plane, unsigned int* bins) {
+__device__ __forceinline__ void color_pixel(const ColorParams& p, const HslBands& bands, long long i, long long plane,
+                                            unsigned int* bins) {
   float v[3] = {p.in[i], p.in[plane + i], p.in[2 * plane + i]};
   if (p.camera_native) {
     v[0] *= p.wb[0];
@@ -52,7 +53,7 @@ __device__ __forceinline__ void color_pixel(const ColorParams& p, long long i, l
     v[1] = p.m[3] * a + p.m[4] * b + p.m[5] * c;
     v[2] = p.m[6] * a + p.m[7] * b + p.m[8] * c;
   }
-  apply_adjustments(p.adj, v);
+  apply_adjustments(p.adj, bands, v);
   float lin[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
@@ -63,27 +64,28 @@ __device__ __forceinline__ void color_pixel(const ColorParams& p, long long i, l
     lin[r] = l;
   }
   // (encoded * 255 + dither).round().clamp(0, 255) with DitherMode::None.
-  float code[3];
-  quantize_srgb3(lin, 255.0f, 0.0f, code);
-  const unsigned char q[3] = {(unsigned char)code[0], (unsigned char)code[1], (unsigned char)code[2]};
+  unsigned q[3];
+  quantize_srgb3<255u>(lin, 0.0f, q);
   const long long y = i / p.W, x = i % p.W;
   unsigned char* o = p.out + y * 3 * p.W + 3 * x;
-  o[0] = q[0];
-  o[1] = q[1];
-  o[2] = q[2];
+  o[0] = (unsigned char)q[0];
+  o[1] = (unsigned char)q[1];
+  o[2] = (unsigned char)q[2];
   atomicAdd(&bins[q[0]], 1u);
   atomicAdd(&bins[256 + q[1]], 1u);
   atomicAdd(&bins[512 + q[2]], 1u);
   atomicAdd(&bins[768 + (2126u * q[0] + 7152u * q[1] + 722u * q[2] + 5000u) / 10000u], 1u);
 }
 
-__global__ void __launch_bounds__(256, 4) color_kernel(const ColorParams p) {
+__global__ void __launch_bounds__(256, 4) color_kernel(const __grid_constant__ ColorParams p) {
   __shared__ unsigned int bins[1024];
+  __shared__ HslBands bands;
+  stage_bands(p.adj, bands);
   for (int k = threadIdx.x; k < 1024; k += blockDim.x) bins[k] = 0;
   __syncthreads();
   const long long plane = (long long)p.W * p.H;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x)
-    color_pixel(p, i, plane, bins);
+    color_pixel(p, bands, i, plane, bins);
   __syncthreads();
   for (int k = threadIdx.x; k < 1024; k += blockDim.x)
     if (bins[k]) atomicAdd(&p.hist[k], (unsigned long long)bins[k]);
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(256) color_batch_kernel(const ColorParams* __r
                                                           const int* __restrict__ block_start, int n) {
   __shared__ unsigned int bins[1024];
   __shared__ ColorParams sp;
+  __shared__ HslBands bands;
   const int b = blockIdx.x;
   int lo = 0, hi = n;
   while (hi - lo > 1) {
@@ -104,12 +107,13 @@ __global__ void __launch_bounds__(256) color_batch_kernel(const ColorParams* __r
     else hi = mid;
   }
   if (threadIdx.x == 0) sp = params[lo];
+  stage_bands(params[lo].adj, bands);
   for (int k = threadIdx.x; k < 1024; k += blockDim.x) bins[k] = 0;
   __syncthreads();
   const long long plane = (long long)sp.W * sp.H;
   const int first = block_start[lo], nb = block_start[lo + 1] - first;
   for (long long i = (long long)(b - first) * blockDim.x + threadIdx.x; i < plane; i += (long long)nb * blockDim.x)
-    color_pixel(sp, i, plane, bins);
+    color_pixel(sp, bands, i, plane, bins);
   __syncthreads();
   for (int k = threadIdx.x; k < 1024; k += blockDim.x)
     if (bins[k]) atomicAdd(&sp.hist[k], (unsigned long long)bins[k]);
