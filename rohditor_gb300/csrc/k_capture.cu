@@ -32,6 +32,7 @@
 #include <mutex>
 #include <vector>
 
+#include "quick_div.cuh"
 #include "rd_internal.cuh"
 #include "tma.cuh"
 
@@ -439,37 +440,7 @@ Status launch_rl_iter(Context& ctx, const float* est, const float* guide, float*
   return Status{};
 }
 
-// ---- RL iteration, constant-lag streaming ------------------------------------
-// The same iteration as rl_stream_kernel for images of at least 256 x 64, with
-// less bookkeeping per row. Each step loads one 8-row estimate block E..E+7 and
-// always advances every stage by 8 rows at fixed lags: blur #1 and the ratio
-// produce rows E-R..E-R+7, blur #2 and the update rows E-2R..E-2R+7. The 2R
-// rows each vertical pass needs from earlier steps (and the estimate values of
-// the update rows) are carried in registers, so every shared-memory access in
-// a step is a per-step base plus a compile-time offset. Rows a segment does not
-// own are computed and dropped instead of being skipped.
-//  * Rows outside the image are mirrored on load (half-sample symmetric, as
-//    the reference samples). The first blur is row-wise, so its mirrored rows
-//    equal the rows they mirror bit for bit; the ratio is not (its vertical
-//    sum would run in reverse order), so the second blur's mirrored rows are
-//    copied from the rows they mirror inside the register window: at the
-//    image top in step R/2 of the first segment, at the bottom in the last
-//    step of the last segment, whose start is aligned so that this step ends
-//    exactly at the last image row. Columns outside the image are handled as
-//    in rl_stream_kernel (mirrored estimate columns, copied ratio columns).
-//  * With tensor maps (rows of a multiple of 16 bytes) the guide rows of a
-//    step (E-2R .. E-R+7) arrive as one tensor copy beside the estimate block,
-//    two steps ahead, and are read from shared memory; rows and columns
-//    outside the image read the fill value 0 and only feed dropped outputs or
-//    ratio columns that are overwritten by their mirrors.
-//  * Horizontal passes run 9-column windows from registers over rows padded
-//    so that every run of a step takes the same path (15 runs cover the 128
-//    blur #1 columns, 14 the strip's output columns; the extra outputs land
-//    in the padding and are never read).
-//  * A sum starts from its first product instead of from zero: every value of
-//    the iteration is positive (estimate >= guide / 2 > 0, ratio >= 0, taps >
-//    0), and 0 + p = p for every such p, so the sums are unchanged.
-// Work item idx -> (strip, segment) for the dynamically scheduled strip
+// Work item idx -> (strip, segment) for the strip
 // kernels: the items of the two edge strips (per-thread copies with mirrored
 // columns, the slowest) are handed out first, then the interior strips', so
 // that the longest items start early and the shorter ones fill in behind them.
@@ -485,6 +456,367 @@ __device__ __forceinline__ void strip_item(int idx, int strips, int segs, int& s
   seg = j / ni;
 }
 
+// ---- RL iteration, a strip of columns per warp -------------------------------
+// The same iteration as rl_stream_kernel for images of at least 256 x 64,
+// without stages in shared memory and without barriers: a warp walks a row segment
+// of a strip of 128 columns, four to a lane, one row at a time, and the whole
+// pipeline (two separable blurs, ratio, update) lives in its registers.
+//  * Horizontal taps come from the neighbouring lanes by shuffles. The margin
+//    lanes of the strip feed the others and store nothing: 112 columns (120 for
+//    R <= 2) are stored of 128.
+//  * A vertical blur keeps partial sums of the 2R outputs that still miss rows:
+//    an arriving row adds its product to each of them (oldest tap first, the
+//    order of the sum over rows), finishes one and starts one. The taps are
+//    symmetric, so R + 1 products a row serve all 2R + 1 sums.
+//  * Sums run in packed pairs of columns (0, 2) and (1, 3).
+//  * Rows arrive by asynchronous copies in a ring that holds what the update,
+//    2R rows behind, still needs; a lane reads only what it copied itself, so
+//    nobody waits for anybody.
+//  * Rows outside the image are mirrored on load (half-sample symmetric, as the
+//    reference samples). The first blur is row-wise across, so its mirrored rows
+//    equal the rows they mirror; the ratio is not (its vertical sum would run in
+//    reverse), so the second blur's mirrored rows are repeated from the blurred
+//    rows they mirror, kept in shared memory at the image's top and bottom.
+//    Columns outside the image: mirrored estimate columns, copied ratio columns.
+//  * A sum starts from its first product instead of from zero: every value of
+//    the iteration is positive (estimate >= guide / 2 > 0, ratio >= 0, taps >
+//    0), and 0 + p = p for every such p, so the sums are unchanged.
+//
+// Measured at 6048 x 4024, R = 3 (radius 0.7): 74 us an iteration, 105 us with
+// the stages in shared memory (four barriers for 8 rows, 108 instructions a
+// pixel against 72). The estimate and the guide read once and the estimate
+// written take 44 us; the separately rounded products and sums (4 passes of 13
+// or 10, the ratio) 43 us of the FP32 pipe with the margins counted. 11648 x
+// 8736: 264 us (360); 512 x 344: 9.7 us (20).
+struct StepImage {
+  const float* est_in;
+  const float* guide;
+  float* est_out;
+  int W, H, strips, segs, items;
+};
+
+template <int R>
+struct StripGeom {
+  static constexpr int MARGIN = (2 * R + 3) / 4;           // lanes at each side that only feed
+  static constexpr int OUT = 4 * (32 - 2 * MARGIN);        // output columns of a strip
+  static constexpr int AHEAD = 3;                          // steps in flight
+  static constexpr int STEPS = 2 * R + AHEAD + 1;          // steps in the ring: of rows o .. o + 2R + AHEAD
+  static constexpr int RESIDENT = R <= 3 ? 16 : 14;        // warps an SM holds: by registers, by the ring at R = 4
+  static_assert(R <= 4, "a window reaches into the next lane only");
+};
+template <int R>
+struct StripRing {
+  float4 step[StripGeom<R>::STEPS][2][32];  // an estimate row and the guide row R above it
+  float4 edge[R + 1][32];  // R rows of the second blur at the image's top or bottom, one ratio row
+};
+
+// A lane's four columns x .. x + 3 of a plane: where a row's start, and the copy
+// of a row's into the lane's place of a ring row (a shared address). VEC: rows
+// start on 16 bytes and W is a multiple of 4. Outside the image the columns
+// mirror.
+struct Columns {
+  const char* base;
+  unsigned pitch;
+  __device__ __forceinline__ const char* row(int y) const { return base + (unsigned long long)(unsigned)y * pitch; }
+};
+template <bool VEC, bool INSIDE>
+__device__ __forceinline__ Columns columns(const float* plane, int x, int W) {
+  return Columns{reinterpret_cast<const char*>(plane + (INSIDE ? x : 0)), 4u * (unsigned)W};
+}
+template <bool VEC, bool INSIDE>
+__device__ __forceinline__ void strip_fetch(unsigned place, const char* row, int x, int W) {
+  if constexpr (VEC && INSIDE) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(place), "l"(row) : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = INSIDE ? j : min(max(x + j, -1 - x - j), 2 * W - 1 - x - j);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(place + 4 * j), "l"(row + 4 * c) : "memory");
+    }
+  }
+}
+template <int OFFSET>
+__device__ __forceinline__ float4 strip_read(unsigned place) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4+%5];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(place), "n"(OFFSET) : "memory");
+  return v;
+}
+__device__ __forceinline__ int mirror_once(int y, int H) {
+  y = max(y, -1 - y);
+  return min(y, 2 * H - 1 - y);
+}
+
+// The four columns of a lane as two packed pairs.
+struct Quad {
+  float2 a, b;
+};
+
+// Horizontal taps of a row.
+template <int R>
+__device__ __forceinline__ Quad strip_blur(const float4 v, const float2 (&k2)[R + 1], float2 z) {
+  const float own[4] = {v.x, v.y, v.z, v.w};
+  float win[4 + 2 * R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    win[j] = __shfl_up_sync(0xffffffffu, own[4 - R + j], 1);
+    win[R + 4 + j] = __shfl_down_sync(0xffffffffu, own[j], 1);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) win[R + j] = own[j];
+  Quad o;
+  o.a = pmul(make_float2(win[0], win[1]), k2[0], z);
+  o.b = pmul(make_float2(win[2], win[3]), k2[0], z);
+#pragma unroll
+  for (int t = 1; t <= 2 * R; ++t) {
+    const float2 k = k2[t <= R ? t : 2 * R - t];
+    o.a = padd(o.a, pmul(make_float2(win[t], win[t + 1]), k, z));
+    o.b = padd(o.b, pmul(make_float2(win[t + 2], win[t + 3]), k, z));
+  }
+  return o;
+}
+
+// One row h into the vertical sums: the finished one is returned.
+template <int R>
+__device__ __forceinline__ float2 strip_feed(float2 (&acc)[2 * R], float2 h, const float2 (&k2)[R + 1], float2 z) {
+  float2 p[R + 1];
+#pragma unroll
+  for (int i = 0; i <= R; ++i) p[i] = pmul(h, k2[i], z);
+  const float2 out = padd(acc[0], p[0]);
+#pragma unroll
+  for (int i = 0; i + 1 < 2 * R; ++i) {
+    const int t = 2 * R - 1 - i;
+    acc[i] = padd(acc[i + 1], p[t <= R ? t : 2 * R - t]);
+  }
+  acc[2 * R - 1] = p[0];
+  return out;
+}
+
+// One work item (a strip and the rows [y0, y1) of segment seg) of one image's
+// iteration. INSIDE: the strip's 128 columns all lie in the image.
+template <int R, bool VEC, bool INSIDE>
+__device__ __forceinline__ void strip_rows(const StepImage& im, int xb, int seg, const float2 (&k2)[R + 1], float2 z,
+                                           StripRing<R>& ring) {
+  using G = StripGeom<R>;
+  constexpr int N2 = 2 * R;
+  const int lane = threadIdx.x;
+  const int W = im.W, H = im.H, x = xb + 4 * lane;
+  const int y0 = (int)((long long)seg * H / im.segs), y1 = (int)((long long)(seg + 1) * H / im.segs);
+  const bool top = y0 == 0, bottom = y1 == H;
+  const bool store = lane >= G::MARGIN && lane < 32 - G::MARGIN && x < W;
+  // Step i brings the estimate row first + i (mirrored outside the image) and
+  // the guide row R above it, AHEAD steps ahead, to a ring. The ratio row r
+  // is R rows behind the estimate row, the output row o R rows behind that.
+  const int first = top ? -R : y0 - N2, r_end = bottom ? H : y1 + R;
+  int r = first + R, o = y0, y_in = first;
+  const int y_last = r_end + R - 1;
+  // Shared addresses of this lane's place in the ring: the step arriving, the
+  // current one, those that brought the estimate and the guide of row o (with
+  // steps y0 - first and y0 + R - first to begin with).
+  constexpr unsigned STEP = sizeof(ring.step[0]), GUIDE = STEP / 2;
+  const unsigned begin = (unsigned)__cvta_generic_to_shared(&ring.step[0][0][lane]), end = begin + G::STEPS * STEP;
+  unsigned in = begin, at = begin, out_e = begin + (y0 - first) % G::STEPS * STEP,
+           out_g = begin + (y0 + R - first) % G::STEPS * STEP;
+  auto next = [&](unsigned& place) {
+    place += STEP;
+    if (place == end) place = begin;
+  };
+  // The last AHEAD fetches repeat the last row, into places nobody reads.
+  const Columns est = columns<VEC, INSIDE>(im.est_in, x, W), guide = columns<VEC, INSIDE>(im.guide, x, W);
+  auto fetch = [&]() {
+    strip_fetch<VEC, INSIDE>(in, est.row(mirror_once(y_in, H)), x, W);
+    strip_fetch<VEC, INSIDE>(in + GUIDE, guide.row(max(y_in - R, 0)), x, W);
+    next(in);
+    y_in = min(y_in + 1, y_last);
+    cp_async_commit();
+  };
+#pragma unroll 1
+  for (int i = 0; i < G::AHEAD; ++i) fetch();
+  float2 va[N2], vb[N2], ua[N2], ub[N2];  // vertical sums of the first and the second blur
+#pragma unroll
+  for (int i = 0; i < N2; ++i) va[i] = vb[i] = ua[i] = ub[i] = make_float2(1.0f, 1.0f);
+  // The first blur: the step's estimate row in, the row R above it out. Every
+  // lane reads what it copied itself, so its own wait is enough.
+  auto blur1 = [&]() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(G::AHEAD - 1) : "memory");
+    const float4 e = strip_read<0>(at);
+    fetch();
+    const Quad h = strip_blur<R>(e, k2, z);
+    return Quad{strip_feed<R>(va, h.a, k2, z), strip_feed<R>(vb, h.b, k2, z)};
+  };
+  auto skip = [&]() {  // a step without a ratio row
+    blur1();
+    next(at);
+  };
+  // The ratio of row r and its horizontal taps.
+  auto ratio = [&](const Quad b) {
+    const float4 gq = strip_read<(int)GUIDE>(at);
+    next(at);
+    // fmaxf(b, FLOOR) equals rmax(b, FLOOR): the floor is not NaN, and a NaN b
+    // gives the floor either way. Both operands are at least 1e-6; those above
+    // 2^60 divide the general way.
+    const float d0 = fmaxf(b.a.x, FLOOR), d1 = fmaxf(b.a.y, FLOOR), d2 = fmaxf(b.b.x, FLOOR), d3 = fmaxf(b.b.y, FLOOR);
+    float4 q = make_float4(quick_div(gq.x, d0), quick_div(gq.y, d1), quick_div(gq.z, d2), quick_div(gq.w, d3));
+    if (!(fmaxf(fmaxf(fmaxf(d0, d1), fmaxf(d2, d3)), fmaxf(fmaxf(gq.x, gq.y), fmaxf(gq.z, gq.w))) <= 0x1p60f))
+      q = make_float4(gq.x / d0, gq.y / d1, gq.z / d2, gq.w / d3);
+    ++r;
+    if (!INSIDE) {
+      // Ratio columns outside the image within R of it take their mirror's value.
+      float4* row = ring.edge[R];
+      row[lane] = q;
+      __syncwarp();
+      auto copied = [&](int c, float v) {
+        return (unsigned)c >= (unsigned)W && c >= -R && c < W + R
+                   ? reinterpret_cast<const float*>(row)[mirror_once(c, W) - xb] : v;
+      };
+      q = make_float4(copied(x, q.x), copied(x + 1, q.y), copied(x + 2, q.z), copied(x + 3, q.w));
+      __syncwarp();
+    }
+    return strip_blur<R>(q, k2, z);
+  };
+  const Columns out = columns<VEC, true>(im.est_out, x, W);
+  auto keep = [&](int row, const Quad h) { ring.edge[row][lane] = make_float4(h.a.x, h.a.y, h.b.x, h.b.y); };
+  auto kept = [&](int row) {
+    const float4 h = ring.edge[row][lane];
+    return Quad{make_float2(h.x, h.y), make_float2(h.z, h.w)};
+  };
+  // The second blur: ratio row in, the finished row R above it out.
+  auto blur2 = [&](const Quad h) { return Quad{strip_feed<R>(ua, h.a, k2, z), strip_feed<R>(ub, h.b, k2, z)}; };
+  // The bounded update of row o. The develop rejects non-finite capture input,
+  // so nothing is NaN here, and min / max give the reference's
+  // compare-and-replace.
+  auto update = [&](const Quad b) {
+    const float4 eo = strip_read<0>(out_e), go = strip_read<(int)GUIDE>(out_g);
+    next(out_e);
+    next(out_g);
+    const float n0 = fminf(fmaxf(eo.x * b.a.x, go.x * 0.5f), go.x * 2.0f);
+    const float n1 = fminf(fmaxf(eo.y * b.a.y, go.y * 0.5f), go.y * 2.0f);
+    const float n2 = fminf(fmaxf(eo.z * b.b.x, go.z * 0.5f), go.z * 2.0f);
+    const float n3 = fminf(fmaxf(eo.w * b.b.y, go.w * 0.5f), go.w * 2.0f);
+    if (store) {
+      float* d = reinterpret_cast<float*>(const_cast<char*>(out.row(o)));
+      if (VEC) {
+        *reinterpret_cast<float4*>(d) = make_float4(n0, n1, n2, n3);
+      } else {
+        d[0] = n0;
+        if (x + 1 < W) d[1] = n1;
+        if (x + 2 < W) d[2] = n2;
+        if (x + 3 < W) d[3] = n3;
+      }
+    }
+    ++o;
+  };
+#pragma unroll 1
+  for (int i = 0; i < N2; ++i) skip();
+  if (top) {
+    // The rows above the image mirror the first R rows.
+#pragma unroll 1
+    for (int i = 0; i < R; ++i) keep(i, ratio(blur1()));
+#pragma unroll 1
+    for (int i = -R; i < R; ++i) blur2(kept(mirror_once(i, H)));
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < N2; ++i) blur2(ratio(blur1()));
+  }
+  const int keep_from = bottom ? H - R : r_end;
+#pragma unroll 1
+  while (r < r_end) {
+    const int row = r;
+    const Quad h = ratio(blur1());
+    if (row >= keep_from) keep(H - 1 - row, h);
+    update(blur2(h));
+  }
+  if (bottom) {
+#pragma unroll 1
+    for (int i = 0; i < R; ++i) update(blur2(kept(i)));
+  }
+}
+template <int R, bool VEC>
+__device__ __forceinline__ void strip_step(const StepImage& im, int item, const float2 (&k2)[R + 1], float2 z,
+                                           StripRing<R>& ring) {
+  int strip, seg;
+  strip_item(item, im.strips, im.segs, strip, seg);
+  const int xb = strip * StripGeom<R>::OUT - 4 * StripGeom<R>::MARGIN;
+  if (xb >= 0 && xb + 128 <= im.W) strip_rows<R, VEC, true>(im, xb, seg, k2, z, ring);
+  else strip_rows<R, VEC, false>(im, xb, seg, k2, z, ring);
+}
+
+template <int R>
+struct StripTaps {
+  float2 k2[R + 1], z;
+  __device__ __forceinline__ explicit StripTaps(const Taps& taps) {
+#pragma unroll
+    for (int k = 0; k <= R; ++k) k2[k] = make_float2(taps.w[k], taps.w[k]);
+    z = make_float2(taps.neg_zero, taps.neg_zero);
+  }
+};
+
+// One warp a block, so that rows, loop counts and row addresses are uniform.
+template <int R, bool VEC>
+__global__ void __launch_bounds__(32, StripGeom<R>::RESIDENT) rl_strip_kernel(const StepImage im, const Taps taps) {
+  __shared__ StripRing<R> ring;
+  const StripTaps<R> t(taps);
+  strip_step<R, VEC>(im, blockIdx.x, t.k2, t.z, ring);
+}
+
+// One iteration of several images in one launch (the batched develop's flat
+// pass): work items image by image in the table's order; first_item[i] is image
+// i's first item (first_item[n] = items). The images share the taps.
+template <int R, bool VEC>
+__global__ void __launch_bounds__(32, StripGeom<R>::RESIDENT)
+    rl_strip_images_kernel(const StepImage* __restrict__ images, const int* __restrict__ first_item, int nimages,
+                           const Taps taps) {
+  __shared__ StripRing<R> ring;
+  const StripTaps<R> t(taps);
+  const int item = blockIdx.x;
+  int lo = 0, hi = nimages;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (first_item[mid] <= item) lo = mid;
+    else hi = mid;
+  }
+  const StepImage im = images[lo];
+  strip_step<R, VEC>(im, item - first_item[lo], t.k2, t.z, ring);
+}
+
+// Images of at least 256 x 64; smaller ones keep rl_stream_kernel, which copes
+// with windows wider than the image.
+bool rl_uses_strip_kernel(int W, int H, int R) { return W >= 256 && H >= 64 && R >= 1 && R <= 4; }
+
+// Row segments of a strip: at least 8 rows each (2R rows of the neighbouring
+// segments are read above and below).
+int strip_segments(int H, int want) { return std::max(1, std::min(want, H / 8)); }
+int strip_count(int W, int R) {
+  const int out = 4 * (32 - 2 * ((2 * R + 3) / 4));
+  return (W + out - 1) / out;
+}
+
+template <int R>
+int strip_slots(int sms) {  // resident warps of the device
+  int occ = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_strip_kernel<R, true>, 32, 0);
+  cudaGetLastError();
+  return std::max(1, occ) * std::max(1, sms);
+}
+
+// Vector loads and stores: 16-byte rows in planes that start on 16 bytes.
+bool strip_vector(const float* planes, int W) { return W % 4 == 0 && (reinterpret_cast<uintptr_t>(planes) & 15) == 0; }
+
+template <int R>
+Status launch_rl_strip(Context& ctx, const float* est, const float* guide, float* out, int W, int H, const Taps& taps,
+                       int want) {
+  const int segs = strip_segments(H, want), strips = strip_count(W, R);
+  const StepImage im{est, guide, out, W, H, strips, segs, strips * segs};
+  // The two estimates and the guide are planes of one allocation.
+  if (strip_vector(est, W) && strip_vector(guide, W) && strip_vector(out, W)) {
+    RD_LAUNCH(ctx, K_RL_ITER, rl_strip_kernel<R, true><<<im.items, 32, 0, ctx.stream>>>(im, taps));
+  } else {
+    RD_LAUNCH(ctx, K_RL_ITER, rl_strip_kernel<R, false><<<im.items, 32, 0, ctx.stream>>>(im, taps));
+  }
+  return Status{};
+}
+
+// ---- work items and runs of the guide and mask kernel ------------------------
 // Next work item of the CTA from the context's counter, broadcast through
 // shared memory; the barrier in front also ends every read of the previous
 // item's shared buffers. Every CTA stops at its first fetch past the last item,
@@ -501,34 +833,6 @@ __device__ __forceinline__ int next_item(unsigned* work, int items, int& s_item)
   __syncthreads();
   return s_item;
 }
-
-template <int R>
-struct StepGeom {
-  static constexpr int QW = 128;         // blur #1 / ratio columns [x0 - R, x0 - R + 128)
-  static constexpr int SW = QW - 2 * R;  // output columns of a strip
-  static constexpr int EW = QW + 2 * R;  // estimate columns [x0 - 2R, x0 - 2R + EW)
-  static constexpr int BH = 8;
-  static constexpr int GH = BH + R;      // guide rows of a step: E-2R .. E-R+7
-  static constexpr int RUN = 9, H1_RUNS = 15, H2_RUNS = 14;
-  static constexpr int PW = 144;                    // row stride of the blur and ratio rows
-  static constexpr int EWP = R <= 3 ? 144 : 176;    // estimate / guide row stride = tensor-copy box width
-  static constexpr int GSLOT = (GH * EWP + 31) & ~31;  // guide slot, a multiple of 128 bytes
-  static_assert(RUN * H1_RUNS >= QW && RUN * H2_RUNS >= SW, "runs cover the rows");
-  static_assert(3 + RUN * H1_RUNS - 1 + 2 * R < EWP, "blur #1 windows stay inside an estimate row");
-  static_assert(RUN * H2_RUNS - 1 + 2 * R < PW && RUN * H1_RUNS <= PW, "blur #2 windows stay inside a ratio row");
-  static_assert(EW + 3 <= EWP && (EWP * 4) % 16 == 0 && (BH * EWP * 4) % 128 == 0, "estimate ring layout");
-  static_assert(H1_RUNS * BH <= 128 && H2_RUNS * BH <= 128, "one run per thread");
-};
-
-template <int R, bool TMA>
-struct __align__(128) StepSmem {
-  using G = StepGeom<R>;
-  float e[3 * G::BH][G::EWP];       // three 8-row estimate blocks (tensor-copy targets)
-  float g[TMA ? 3 : 1][G::GSLOT];   // three guide slots (tensor-copy targets)
-  float t[G::BH][G::PW];            // blur #1 rows E..E+7, then blur #2 rows E-R..E-R+7
-  float q[G::BH][G::PW];            // ratio rows E-R..E-R+7
-  unsigned long long bar[3];
-};
 
 template <int R, int RUN>
 __device__ __forceinline__ void hrun_full(const float* __restrict__ src, float* __restrict__ dst,
@@ -553,395 +857,6 @@ __device__ __forceinline__ void hrun_full(const float* __restrict__ src, float* 
     for (int t = 1; t < T; ++t) v += win[j + t] * w[t];
     dst[j] = v;
   }
-}
-
-// The vertical tap sums of BH consecutive rows from a window of BH + 2R rows:
-// out[j] = sum_t win[j + t] w[t], rows j and j + BH/2 in the two lanes.
-template <int R, int BH>
-__device__ __forceinline__ void vsum_packed(const float (&win)[BH + 2 * R], const float2 (&w2)[2 * R + 1], float2 z,
-                                            float (&out)[BH]) {
-  constexpr int T = 2 * R + 1, HALF = BH / 2;
-  static_assert(BH % 2 == 0, "rows pair up");
-#pragma unroll
-  for (int j = 0; j < HALF; ++j) {
-    float2 v = pmul(make_float2(win[j], win[j + HALF]), w2[0], z);
-#pragma unroll
-    for (int t = 1; t < T; ++t) v = padd(v, pmul(make_float2(win[j + t], win[j + HALF + t]), w2[t], z));
-    out[j] = v.x;
-    out[j + HALF] = v.y;
-  }
-}
-
-// Row segments: 8-row units spread evenly; every boundary lies at
-// H + 4R (mod 8) so that the last segment's final step ends at row H - 1.
-// Segment s covers [seg_row(s), seg_row(s + 1)).
-struct StepSegments {
-  int q, rem, r8, segs;
-};
-__host__ __device__ __forceinline__ int seg_row(const StepSegments& sg, int s, int H) {
-  if (s <= 0) return 0;
-  if (s >= sg.segs) return H;
-  return sg.r8 + 8 * (s * sg.q + min(s, sg.rem));
-}
-StepSegments step_segments(int H, int R, int want) {
-  const int m = (4 * R) % 8;
-  const int n8 = (H - m) / 8;
-  const int segs = std::max(2, std::min(want, n8));
-  return {n8 / segs, n8 % segs, (H - m) % 8, segs};
-}
-
-// One image of an iteration launch: its estimate (in and out) and guide
-// planes, its size, strips, row segments and work items, and the tensor maps
-// of its estimate and guide planes (null without tensor copies).
-struct StepImage {
-  const float* est_in;
-  const float* guide;
-  float* est_out;
-  int W, H, strips, items;
-  StepSegments sg;
-  const CUtensorMap* est_map;
-  const CUtensorMap* guide_map;
-};
-
-// A thread's part of an iteration launch: the taps (scalar and packed), the
-// -0.0 addend of the packed products, and the run it computes in each
-// horizontal pass (row, first column).
-template <int R>
-struct StepThread {
-  using G = StepGeom<R>;
-  float w[2 * R + 1];
-  float2 w2[2 * R + 1];
-  float2 z2;
-  bool h1_on, h2_on;
-  int h1_row, h1_col, h2_row, h2_col;
-  __device__ __forceinline__ explicit StepThread(const Taps& taps) {
-#pragma unroll
-    for (int k = 0; k < 2 * R + 1; ++k) {
-      w[k] = taps.w[k];
-      w2[k] = make_float2(taps.w[k], taps.w[k]);
-    }
-    z2 = make_float2(taps.neg_zero, taps.neg_zero);
-    const int tid = threadIdx.x;
-    h1_on = tid < G::H1_RUNS * G::BH;
-    h2_on = tid < G::H2_RUNS * G::BH;
-    h1_row = tid / G::H1_RUNS;
-    h1_col = (tid % G::H1_RUNS) * G::RUN;
-    h2_row = tid / G::H2_RUNS;
-    h2_col = (tid % G::H2_RUNS) * G::RUN;
-  }
-};
-
-// One work item (a strip and a row segment) of one image's iteration. Every
-// thread of the CTA calls it.
-template <int R, bool TMA>
-__device__ __forceinline__ void step_item(StepSmem<R, TMA>& S, const StepImage& im, int item, const StepThread<R>& th,
-                                          CopyWaits& cw) {
-  using G = StepGeom<R>;
-  constexpr int SW = G::SW, BH = G::BH, N2 = 2 * R;
-  const int tid = threadIdx.x;
-  const float(&w)[2 * R + 1] = th.w;
-  const float2(&w2)[2 * R + 1] = th.w2;
-  const float2 z2 = th.z2;
-  const bool h1_on = th.h1_on, h2_on = th.h2_on;
-  const int h1_row = th.h1_row, h1_col = th.h1_col, h2_row = th.h2_row, h2_col = th.h2_col;
-  const float* __restrict__ est_in = im.est_in;
-  const float* __restrict__ guide = im.guide;
-  float* __restrict__ est_out = im.est_out;
-  const int W = im.W, H = im.H, strips = im.strips;
-  const StepSegments sg = im.sg;
-  int strip, seg;
-  strip_item(item, strips, sg.segs, strip, seg);
-  const int x0 = strip * SW;
-  const int y0 = seg_row(sg, seg, H), y1 = seg_row(sg, seg + 1, H);
-  const int E0 = y0 - N2;
-  const int nsteps = (y1 - y0 + 2 * N2 - BH + 7) / BH + 1;
-  const bool inside = x0 - N2 >= 0 && x0 - N2 + G::EW <= W;
-  const bool tma_strip = TMA && inside;
-  const bool edge_q = x0 < R || x0 + SW + R > W;
-  const int xal = (x0 - N2) & ~3;  // rounds down, also below 0
-  const int rem = TMA ? (x0 - N2) - xal : 0;
-  // Guide boxes stay inside the image columns (a box crossing the image edge
-  // takes the tensor unit much longer); reads shift by xal - gx. Columns the
-  // shifted box misses lie outside the image and only feed ratio columns
-  // that are overwritten by their mirrors and outputs that are not stored.
-  const int gx = TMA ? min(max(xal, 0), W - G::EWP) : 0;
-  const int xa = x0 - N2 + tid, xb = xa + 128;
-  const int sxa = (unsigned)xa < (unsigned)W ? xa : mirror_half(xa, W);
-  const bool has_b = tid + 128 < G::EW;
-  const int sxb = has_b ? ((unsigned)xb < (unsigned)W ? xb : mirror_half(xb, W)) : 0;
-  // Step k's estimate block (rows [E0 + 8k, +8)) goes to ring block k % 3, by
-  // one tensor copy when the rows and the window lie inside the image, else
-  // by per-thread copies with rows and columns mirrored into the image; its
-  // guide rows go to guide slot k % 3 by one tensor copy.
-  auto e_by_tma = [&](int k) {
-    const int r0 = E0 + BH * k;
-    return tma_strip && r0 >= 0 && r0 + BH <= H;
-  };
-  auto issue = [&](int k) {
-    if (k >= nsteps) return;
-    const int r0 = E0 + BH * k, b = k % 3;
-    const bool et = e_by_tma(k);
-    if (TMA && cw.issue_block(b) && tid == 0) {
-      fence_proxy_async();
-      mbar_expect_tx(&S.bar[b], (et ? BH * G::EWP * sizeof(float) : 0) + G::GH * G::EWP * sizeof(float));
-      if (et) tma_load_2d(S.e[b * BH], im.est_map, xal, r0, &S.bar[b]);
-      tma_load_2d(S.g[b], im.guide_map, gx, r0 - N2, &S.bar[b]);
-    }
-    if (et) return;
-#pragma unroll
-    for (int j = 0; j < BH; ++j) {
-      const float* src = est_in + (long long)mirror_row(r0 + j, H) * W;
-      float* dst = S.e[b * BH + j] + rem;
-      cp_async4(dst + tid, src + sxa);
-      if (has_b) cp_async4(dst + tid + 128, src + sxb);
-    }
-  };
-  issue(0);
-  cp_async_commit();
-  issue(1);
-  cp_async_commit();
-  // Carried rows: blur #1 rows [E-2R, E), blur #2 rows [E-3R, E-R), estimate
-  // rows [E-2R, E) of this thread's output column.
-  float c1[N2], c2[N2], ed[N2];
-#pragma unroll
-  for (int i = 0; i < N2; ++i) c1[i] = c2[i] = ed[i] = 1.0f;
-  const int xq = x0 - R + tid, xo = x0 + tid;
-  const bool okq = (unsigned)xq < (unsigned)W;
-  const bool oko = tid < SW && xo < W;
-  for (int k = 0; k < nsteps; ++k) {
-    const int E = E0 + BH * k;
-    // Without tensor maps: guide values of the ratio rows and of the update rows.
-    float gq[BH], go[BH];
-    if (!TMA) {
-#pragma unroll
-      for (int j = 0; j < BH; ++j) {
-        const int rq = E - R + j, ro = E - N2 + j;
-        gq[j] = okq && (unsigned)rq < (unsigned)H ? __ldg(guide + (long long)rq * W + xq) : 0.0f;
-        go[j] = oko && ro >= y0 && ro < y1 ? __ldg(guide + (long long)ro * W + xo) : 0.0f;
-      }
-    }
-    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    if (TMA) cw.wait(&S.bar[k % 3], k % 3);
-    __syncthreads();
-    // Block k + 2 reuses the slots of block k - 1, whose estimate rows were
-    // last read before the second barrier of step k - 1 and whose guide rows
-    // before the barrier above.
-    issue(k + 2);
-    cp_async_commit();
-    const float* eb = S.e[(k % 3) * BH] + rem;
-    const float* gb = S.g[TMA ? k % 3 : 0] + rem + (xal - gx);
-    // 1. blur #1, horizontal: rows E..E+7, columns x0-R .. x0-R+134
-    if (h1_on) hrun_full<R, G::RUN>(eb + h1_row * G::EWP + h1_col, S.t[h1_row] + h1_col, w, w2, z2);
-    float ec[BH];
-#pragma unroll
-    for (int j = 0; j < BH; ++j) ec[j] = eb[j * G::EWP + tid + N2];
-    __syncthreads();
-    // 2. blur #1, vertical, and the ratio: rows E-R .. E-R+7, column x0-R+tid
-    {
-      float win[BH + N2];
-#pragma unroll
-      for (int i = 0; i < N2; ++i) win[i] = c1[i];
-#pragma unroll
-      for (int j = 0; j < BH; ++j) win[N2 + j] = S.t[j][tid];
-      float bs[BH];
-      vsum_packed<R, BH>(win, w2, z2, bs);
-#pragma unroll
-      for (int j = 0; j < BH; ++j) {
-        const float b = bs[j];
-        const float g = TMA ? gb[(R + j) * G::EWP + R + tid] : gq[j];
-        // fmaxf(b, FLOOR) equals rmax(b, FLOOR): the floor is not NaN, and
-        // a NaN b gives the floor either way.
-        S.q[j][tid] = g / fmaxf(b, FLOOR);
-      }
-#pragma unroll
-      for (int i = 0; i < N2; ++i) c1[i] = win[BH + i];
-    }
-    __syncthreads();
-    if (edge_q) {
-      // Ratio columns outside the image within R of it take their mirror's value.
-      if ((unsigned)xq >= (unsigned)W && xq >= -R && xq < W + R) {
-        const int src = mirror_half(xq, W) - (x0 - R);
-#pragma unroll
-        for (int j = 0; j < BH; ++j) S.q[j][tid] = S.q[j][src];
-      }
-      __syncthreads();
-    }
-    // 3. blur #2, horizontal: rows E-R .. E-R+7, output columns (over blur #1,
-    //    whose rows every thread has read before the barrier above)
-    if (h2_on) hrun_full<R, G::RUN>(S.q[h2_row] + h2_col, S.t[h2_row] + h2_col, w, w2, z2);
-    __syncthreads();
-    // 4. blur #2, vertical, and the bounded update: rows E-2R .. E-2R+7
-    {
-      float win[BH + N2];
-#pragma unroll
-      for (int i = 0; i < N2; ++i) win[i] = c2[i];
-#pragma unroll
-      for (int j = 0; j < BH; ++j) win[N2 + j] = S.t[j][tid];
-#pragma unroll
-      for (int i = 0; i < N2; ++i) c2[i] = win[BH + i];
-      if (y0 == 0 && k == R / 2) {
-        // Window position p holds row E - 3R + p; rows -1 .. -R take rows 0 .. R-1.
-        constexpr int P0 = 5 * R - 8 * (R / 2);
-#pragma unroll
-        for (int i = 1; i <= R; ++i) win[P0 - i] = win[P0 + i - 1];
-      }
-      if (y1 == H && k == nsteps - 1) {
-        // This step ends at row H - 1: rows H .. H+R-1 take rows H-1 .. H-R.
-#pragma unroll
-        for (int i = 0; i < R; ++i) win[BH + R + i] = win[BH + R - 1 - i];
-      }
-      if (oko && E - N2 + BH > y0) {
-        float* po = est_out + (long long)(E - N2) * W + xo;
-        float eo[BH];
-        float bs[BH];
-        vsum_packed<R, BH>(win, w2, z2, bs);
-#pragma unroll
-        for (int j = 0; j < BH; ++j) {
-          const float b = bs[j];
-          const float e = (j < N2 ? ed[j] : ec[j - N2]) * b;
-          const float g = TMA ? gb[j * G::EWP + N2 + tid] : go[j];
-          // The develop rejects non-finite capture input, so e is never NaN
-          // here, and min / max give the reference's compare-and-replace.
-          eo[j] = fminf(fmaxf(e, g * 0.5f), g * 2.0f);
-        }
-        if (E - N2 >= y0 && E - N2 + BH <= y1) {
-#pragma unroll
-          for (int j = 0; j < BH; ++j) {
-            *po = eo[j];
-            po += W;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < BH; ++j) {
-            const int o = E - N2 + j;
-            if (o >= y0 && o < y1) *po = eo[j];
-            po += W;
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < N2; ++i) ed[i] = ec[BH - N2 + i];
-  }
-}
-
-template <int R, bool TMA>
-__global__ void __launch_bounds__(128, 5) rl_step_kernel(const float* __restrict__ est_in,
-                                                          const float* __restrict__ guide,
-                                                          float* __restrict__ est_out, int W, int H, int strips,
-                                                          const StepSegments sg, int items, const Taps taps,
-                                                          const __grid_constant__ CUtensorMap est_map,
-                                                          const __grid_constant__ CUtensorMap guide_map,
-                                                          unsigned* work, unsigned* error, unsigned wait_tries,
-                                                          int withhold) {
-  extern __shared__ __align__(128) float4 rl_step_raw[];
-  StepSmem<R, TMA>& S = *reinterpret_cast<StepSmem<R, TMA>*>(rl_step_raw);
-  const StepThread<R> th(taps);
-  if (TMA && threadIdx.x == 0) {
-    for (int b = 0; b < 3; ++b) mbar_init(&S.bar[b]);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncthreads();
-  CopyWaits cw(wait_tries, TMA && withhold != 0, error);
-  const StepImage im{est_in, guide, est_out, W, H, strips, items, sg, &est_map, &guide_map};
-  __shared__ int s_item;
-  for (int item = next_item(work, items, s_item); item < items; item = next_item(work, items, s_item))
-    step_item<R, TMA>(S, im, item, th, cw);
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (TMA) cw.drain(S.bar, 3);
-}
-
-// One iteration of several images in one launch (the batched develop's flat
-// pass): work items of every image from one counter, image by image in the
-// table's order; first_item[i] is image i's first item (first_item[n] = items).
-// The images share the taps; each brings its own planes, size and tensor maps
-// (kept in global memory).
-template <int R, bool TMA>
-__global__ void __launch_bounds__(128, 5) rl_step_images_kernel(const StepImage* __restrict__ images,
-                                                                 const int* __restrict__ first_item, int nimages,
-                                                                 int items, const Taps taps, unsigned* work,
-                                                                 unsigned* error, unsigned wait_tries, int withhold) {
-  extern __shared__ __align__(128) float4 rl_step_raw[];
-  StepSmem<R, TMA>& S = *reinterpret_cast<StepSmem<R, TMA>*>(rl_step_raw);
-  const StepThread<R> th(taps);
-  if (TMA && threadIdx.x == 0) {
-    for (int b = 0; b < 3; ++b) mbar_init(&S.bar[b]);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
-  __syncthreads();
-  CopyWaits cw(wait_tries, TMA && withhold != 0, error);
-  __shared__ int s_item, s_local;
-  __shared__ StepImage s_im;
-  for (;;) {
-    // The barrier in front ends every read of the previous item's buffers.
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const unsigned v = atomicAdd(work, 1u);
-      if (v == (unsigned)items + gridDim.x - 1u) atomicExch(work, 0u);
-      s_item = (int)v;
-      if ((int)v < items) {
-        int lo = 0, hi = nimages;
-        while (hi - lo > 1) {
-          const int mid = (lo + hi) >> 1;
-          if (first_item[mid] <= (int)v) lo = mid;
-          else hi = mid;
-        }
-        s_im = images[lo];
-        s_local = (int)v - first_item[lo];
-      }
-    }
-    __syncthreads();
-    if (s_item >= items) break;
-    const StepImage im = s_im;
-    step_item<R, TMA>(S, im, s_local, th, cw);
-  }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-  if (TMA) cw.drain(S.bar, 3);
-}
-
-// The constant-lag kernel serves images of at least 256 x 64; smaller ones
-// keep the per-step bookkeeping of rl_stream_kernel.
-bool rl_uses_step_kernel(int W, int H, int R) { return W >= 256 && H >= 64 && R >= 1 && R <= 4; }
-
-template <int R, bool TMA>
-int step_occupancy() {
-  int occ = 0;
-  const size_t smem = sizeof(StepSmem<R, TMA>);
-  cudaFuncSetAttribute(rl_step_kernel<R, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_step_kernel<R, TMA>, 128, smem);
-  cudaGetLastError();
-  return std::max(1, occ);
-}
-
-template <int R, bool TMA>
-Status launch_rl_step_t(Context& ctx, const float* est, const float* guide, float* out, int W, int H,
-                        const Taps& taps, const CUtensorMap* est_map, const CUtensorMap* guide_map, int segs) {
-  using G = StepGeom<R>;
-  const size_t smem = sizeof(StepSmem<R, TMA>);
-  RD_CUDA_TRY(cudaFuncSetAttribute(rl_step_kernel<R, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int occ = 0;
-  RD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_step_kernel<R, TMA>, 128, smem));
-  const int sms = ctx.sm_count > 0 ? ctx.sm_count : 152;
-  const int slots = std::max(1, occ) * sms;
-  const int strips = (W + G::SW - 1) / G::SW;
-  const StepSegments sg = step_segments(H, R, segs);
-  const int items = strips * sg.segs;
-  const int grid = std::min(items, slots);
-  CUtensorMap none{};
-  RD_LAUNCH(ctx, K_RL_ITER, rl_step_kernel<R, TMA><<<grid, 128, smem, ctx.stream>>>(
-                                est, guide, out, W, H, strips, sg, items, taps, est_map ? *est_map : none,
-                                guide_map ? *guide_map : none, ctx.d_work, ctx.d_error,
-                                ctx.wait_limit ? ctx.wait_limit : RL_DEFAULT_WAIT_TRIES,
-                                ctx.wait_withhold == RD_WAIT_RL_COPY ? 1 : 0));
-  return Status{};
-}
-
-template <int R>
-Status launch_rl_step(Context& ctx, const float* est, const float* guide, float* out, int W, int H, const Taps& taps,
-                      const CUtensorMap* est_map, const CUtensorMap* guide_map, int segs) {
-  if (est_map && guide_map)
-    return launch_rl_step_t<R, true>(ctx, est, guide, out, W, H, taps, est_map, guide_map, segs);
-  return launch_rl_step_t<R, false>(ctx, est, guide, out, W, H, taps, nullptr, nullptr, segs);
 }
 
 // ---- guide and mask, streamed down column strips ---------------------------
@@ -1392,24 +1307,25 @@ std::mutex g_rl_tune_mutex;
 std::map<RlShape, RlChoice> g_rl_tuned;
 
 // The occupancy heuristic: one round of (strip, segment) items over all
-// resident CTAs, each segment at least 32 rows (vertical halos) and at most
-// 512 (more rounds).
+// resident warps or CTAs. The strip kernel's segments go down to 8 rows: a small
+// image is a matter of latency, and an iteration at 512 x 344 takes 9.7 us with
+// 43 segments of 8 rows, 11.8 with 21, 16.4 with 10. rl_stream_kernel's have at
+// least 32 rows (vertical halos) and at most 512 (more rounds).
 int rl_default_segments(int W, int H, int R, int sms) {
+  if (rl_uses_strip_kernel(W, H, R)) {
+    const int slots = R == 1 ? strip_slots<1>(sms) : R == 2 ? strip_slots<2>(sms) : R == 3 ? strip_slots<3>(sms)
+                                                                                    : strip_slots<4>(sms);
+    return strip_segments(H, std::max(1, slots / strip_count(W, R)));
+  }
   int occ = 0;
   size_t smem = 0;
-  if (rl_uses_step_kernel(W, H, R)) R += 4;  // cases 5..8: the constant-lag kernel (tensor-copy form)
   switch (R) {
-    case 5: occ = step_occupancy<1, true>(); break;
-    case 6: occ = step_occupancy<2, true>(); break;
-    case 7: occ = step_occupancy<3, true>(); break;
-    case 8: occ = step_occupancy<4, true>(); break;
     case 1: smem = sizeof(StreamSmem<1>); cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_stream_kernel<1>, 128, smem); break;
     case 2: smem = sizeof(StreamSmem<2>); cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_stream_kernel<2>, 128, smem); break;
     case 3: smem = sizeof(StreamSmem<3>); cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_stream_kernel<3>, 128, smem); break;
     default: smem = sizeof(StreamSmem<4>); cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_stream_kernel<4>, 128, smem); break;
   }
   cudaGetLastError();
-  if (R > 4) R -= 4;
   const int slots = std::max(1, occ) * std::max(1, sms);
   const int strips = (W + (128 - 2 * R) - 1) / (128 - 2 * R);
   const int per_round = std::max(1, slots / strips);
@@ -1419,11 +1335,11 @@ int rl_default_segments(int W, int H, int R, int sms) {
 }
 
 // Candidate segment counts around the heuristic's (each segment >= 32 rows):
-// fewer, equal and several times more work items than resident CTAs.
+// one, two and three rounds of work items.
 std::vector<int> rl_candidates(int H, int d) {
   std::vector<int> c{d};
-  for (int v : {2 * d, 3 * d, 4 * d, 6 * d, std::max(1, d / 2)})
-    if (H / v >= 32 && std::find(c.begin(), c.end(), v) == c.end()) c.push_back(v);
+  for (int v : {2 * d, 3 * d})
+    if (H / v >= 32) c.push_back(v);
   return c;
 }
 
@@ -1460,12 +1376,6 @@ void resolve_rl_tuning(Context& ctx) {
 
 namespace {
 
-// Estimate-ring box width (floats) of the kernel that runs an iteration.
-int rl_box_width(int W, int H, int R) {
-  if (!rl_uses_step_kernel(W, H, R)) return StreamGeom<1>::EWP;
-  return R <= 3 ? StepGeom<1>::EWP : StepGeom<4>::EWP;
-}
-
 // Tensor map of one f32 plane for the estimate ring's box_w x 8 boxes; false
 // when TMA cannot address it (row stride not a multiple of 16 bytes, or no
 // encoder).
@@ -1475,13 +1385,13 @@ bool make_plane_map(CUtensorMap* map, const float* plane, int W, int H, int box_
 }
 
 Status rl_iteration(Context& ctx, int r, const Taps& taps, const float* est, const float* guide, float* out, int W,
-                    int H, const CUtensorMap* est_map, const CUtensorMap* guide_map, int segs) {
-  if (rl_uses_step_kernel(W, H, r)) {
+                    int H, const CUtensorMap* est_map, int segs) {
+  if (rl_uses_strip_kernel(W, H, r)) {
     switch (r) {
-      case 1: return launch_rl_step<1>(ctx, est, guide, out, W, H, taps, est_map, guide_map, segs);
-      case 2: return launch_rl_step<2>(ctx, est, guide, out, W, H, taps, est_map, guide_map, segs);
-      case 3: return launch_rl_step<3>(ctx, est, guide, out, W, H, taps, est_map, guide_map, segs);
-      case 4: return launch_rl_step<4>(ctx, est, guide, out, W, H, taps, est_map, guide_map, segs);
+      case 1: return launch_rl_strip<1>(ctx, est, guide, out, W, H, taps, segs);
+      case 2: return launch_rl_strip<2>(ctx, est, guide, out, W, H, taps, segs);
+      case 3: return launch_rl_strip<3>(ctx, est, guide, out, W, H, taps, segs);
+      case 4: return launch_rl_strip<4>(ctx, est, guide, out, W, H, taps, segs);
       default: break;
     }
   }
@@ -1753,15 +1663,12 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
     st = rl_prep(ctx, r, taps, rgb, plane, detail.ceilings, detail.noise_protection, guide, mask, W, H,
                  rgb_tma ? &rgb_map : nullptr);
     // Tensor maps of the three planes an iteration can read (guide, then the
-    // ping-pong estimates), for the TMA-fed estimate ring.
+    // ping-pong estimates), for the TMA-fed estimate ring of small images.
     CUtensorMap maps[3];
-    const int box_w = rl_box_width(W, H, r);
-    const bool tma = make_plane_map(&maps[0], guide, W, H, box_w) && make_plane_map(&maps[1], est_buf[0], W, H, box_w) &&
-                     make_plane_map(&maps[2], est_buf[1], W, H, box_w);
+    const int box_w = StreamGeom<1>::EWP;
+    const bool tma = !rl_uses_strip_kernel(W, H, r) && make_plane_map(&maps[0], guide, W, H, box_w) &&
+                     make_plane_map(&maps[1], est_buf[0], W, H, box_w) && make_plane_map(&maps[2], est_buf[1], W, H, box_w);
     const CUtensorMap* in_map = tma ? &maps[0] : nullptr;
-    // The constant-lag kernel also reads each step's guide rows (8 + R) by tensor copy.
-    CUtensorMap guide_map;
-    const bool guide_tma = tma && rl_uses_step_kernel(W, H, r) && make_plane_map(&guide_map, guide, W, H, box_w, 8 + r);
     // Launch shape: the tuned segment count of this image shape, or a tuning
     // run over the candidates (not while the stream is being captured).
     const RlShape shape{W, H, r};
@@ -1796,8 +1703,7 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
         }
         cudaEventRecord(a, ctx.stream);
       }
-      st = rl_iteration(ctx, r, taps, est, guide, est_buf[it & 1], W, H, in_map, guide_tma ? &guide_map : nullptr,
-                        s_it);
+      st = rl_iteration(ctx, r, taps, est, guide, est_buf[it & 1], W, H, in_map, s_it);
       if (timed) {
         cudaEventRecord(b, ctx.stream);
         ctx.tune_runs.push_back({s_it, {a, b}});
@@ -1828,52 +1734,39 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
 // ---- capture sharpening of several images at once ---------------------------
 namespace {
 
-template <int R, bool TMA>
-Status launch_rl_step_images(Context& ctx, const StepImage* d_images, const int* d_first, int nimages, int items,
-                             const Taps& taps) {
-  const size_t smem = sizeof(StepSmem<R, TMA>);
-  RD_CUDA_TRY(
-      cudaFuncSetAttribute(rl_step_images_kernel<R, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int occ = 0;
-  RD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_step_images_kernel<R, TMA>, 128, smem));
-  const int sms = ctx.sm_count > 0 ? ctx.sm_count : 152;
-  const int grid = std::min(items, std::max(1, occ) * sms);
+template <int R, bool VEC>
+Status launch_rl_strip_images(Context& ctx, const StepImage* d_images, const int* d_first, int nimages, int items,
+                              const Taps& taps) {
   RD_LAUNCH(ctx, K_RL_ITER,
-            rl_step_images_kernel<R, TMA><<<grid, 128, smem, ctx.stream>>>(
-                d_images, d_first, nimages, items, taps, ctx.d_work, ctx.d_error,
-                ctx.wait_limit ? ctx.wait_limit : RL_DEFAULT_WAIT_TRIES, ctx.wait_withhold == RD_WAIT_RL_COPY ? 1 : 0));
+            rl_strip_images_kernel<R, VEC><<<items, 32, 0, ctx.stream>>>(d_images, d_first, nimages, taps));
   return Status{};
 }
 
-Status rl_step_images(Context& ctx, int r, bool tma, const StepImage* d_images, const int* d_first, int nimages,
-                      int items, const Taps& taps) {
+Status rl_strip_images(Context& ctx, int r, bool vec, const StepImage* d_images, const int* d_first, int nimages,
+                       int items, const Taps& taps) {
   switch (r) {
-#define RD_STEP_IMAGES_CASE(RR)                                                                       \
+#define RD_STRIP_IMAGES_CASE(RR)                                                                       \
   case RR:                                                                                            \
-    return tma ? launch_rl_step_images<RR, true>(ctx, d_images, d_first, nimages, items, taps)        \
-               : launch_rl_step_images<RR, false>(ctx, d_images, d_first, nimages, items, taps);
-    RD_STEP_IMAGES_CASE(1)
-    RD_STEP_IMAGES_CASE(2)
-    RD_STEP_IMAGES_CASE(3)
-    RD_STEP_IMAGES_CASE(4)
-#undef RD_STEP_IMAGES_CASE
+    return vec ? launch_rl_strip_images<RR, true>(ctx, d_images, d_first, nimages, items, taps)        \
+               : launch_rl_strip_images<RR, false>(ctx, d_images, d_first, nimages, items, taps);
+    RD_STRIP_IMAGES_CASE(1)
+    RD_STRIP_IMAGES_CASE(2)
+    RD_STRIP_IMAGES_CASE(3)
+    RD_STRIP_IMAGES_CASE(4)
+#undef RD_STRIP_IMAGES_CASE
     default:
       return Status{RD_INVALID_INPUT, "capture radius outside 1..4"};
   }
 }
 
-// Per image of run_capture_images: its RL planes, taps and step geometry, and
-// the device copies of its four tensor maps (guide, the two estimates, and
-// the guide for the step kernel's 8 + R row boxes).
+// Per image of run_capture_images: its RL planes, taps and work items.
 struct CapturePlanes {
   int job = -1, r = 0, iterations = 0;
   Taps taps{};
   float* planes = nullptr;
   size_t bytes = 0;
-  bool tma = false;
-  CUtensorMap maps[4];
-  StepSegments sg{};
-  int strips = 0, items = 0;
+  bool vec = false;
+  int segs = 0;
 };
 
 }  // namespace
@@ -1882,7 +1775,7 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
   std::vector<CapturePlanes> prepared;
   const int sms = ctx.sm_count > 0 ? ctx.sm_count : 152;
   // 1. Settings, planes and the guide / mask pass, image by image; images the
-  //    step kernel does not serve take the per-image path whole.
+  //    strip kernel does not serve take the per-image path whole.
   for (int j = 0; j < n; ++j) {
     CaptureJob& job = jobs[j];
     const rd_detail_desc& d = job.detail;
@@ -1893,7 +1786,7 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
     const int ntaps = gaussian_kernel(d.radius, cp.taps.w, MAX_TAPS);
     cp.taps.neg_zero = -0.0f;
     cp.r = ntaps / 2;
-    if (ntaps < 0 || !rl_uses_step_kernel(W, H, cp.r) || d.iterations < 1) {
+    if (ntaps < 0 || !rl_uses_strip_kernel(W, H, cp.r) || d.iterations < 1) {
       job.st = run_capture(ctx, job.rgb, W, H, d);
       continue;
     }
@@ -1926,11 +1819,7 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
       device_free(ctx, cp.planes, cp.bytes);
       continue;
     }
-    const int box_w = rl_box_width(W, H, cp.r);
-    cp.tma = make_plane_map(&cp.maps[0], guide, W, H, box_w) &&
-             make_plane_map(&cp.maps[1], cp.planes + 2 * plane, W, H, box_w) &&
-             make_plane_map(&cp.maps[2], cp.planes + 3 * plane, W, H, box_w) &&
-             make_plane_map(&cp.maps[3], guide, W, H, box_w, 8 + cp.r);
+    cp.vec = strip_vector(cp.planes, W);
     int segs = 0;
     {
       std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
@@ -1938,11 +1827,11 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
       if (it != g_rl_tuned.end()) segs = it->second.segs;
     }
     if (segs == 0) segs = rl_default_segments(W, H, cp.r, sms);
-    cp.sg = step_segments(H, cp.r, segs);
+    cp.segs = strip_segments(H, segs);
     cp.iterations = d.iterations;
     prepared.push_back(cp);
   }
-  // 2. The iterations: images with the same taps and tensor-copy ability
+  // 2. The iterations: images with the same taps and row alignment
   //    share one launch per iteration; an image leaves after its last one.
   Status st;
   std::vector<bool> done(prepared.size(), false);
@@ -1950,34 +1839,29 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
     if (done[g]) continue;
     std::vector<size_t> group;
     for (size_t k = g; k < prepared.size(); ++k)
-      if (!done[k] && prepared[k].r == prepared[g].r && prepared[k].tma == prepared[g].tma &&
+      if (!done[k] && prepared[k].r == prepared[g].r && prepared[k].vec == prepared[g].vec &&
           std::memcmp(prepared[k].taps.w, prepared[g].taps.w, sizeof(float) * (2 * prepared[g].r + 1)) == 0) {
         group.push_back(k);
         done[k] = true;
       }
     const int r = prepared[g].r;
-    const bool tma = prepared[g].tma;
+    const bool vec = prepared[g].vec;
     int max_k = 0;
     for (size_t k : group) max_k = std::max(max_k, prepared[k].iterations);
-    // Device tables: the group's tensor maps, then per iteration the image
-    // table and its first-item offsets.
-    const size_t map_bytes = sizeof(CUtensorMap) * 4 * group.size();
+    // Device tables: per iteration the image table and its first-item offsets.
     const size_t img_bytes = (sizeof(StepImage) * group.size() + 63) & ~(size_t)63;
     const size_t first_bytes = (sizeof(int) * (group.size() + 1) + 63) & ~(size_t)63;
-    const size_t table_bytes = map_bytes + (size_t)max_k * (img_bytes + first_bytes);
+    const size_t table_bytes = (size_t)max_k * (img_bytes + first_bytes);
     void* t = nullptr;
     st = device_alloc(ctx, table_bytes + 64, &t);
     if (!st.ok()) break;
     unsigned char* tb =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(t) + 63) & ~static_cast<uintptr_t>(63));
     std::vector<unsigned char> host(table_bytes, 0);
-    const CUtensorMap* d_maps = reinterpret_cast<const CUtensorMap*>(tb);
-    for (size_t i = 0; i < group.size(); ++i)
-      std::memcpy(host.data() + sizeof(CUtensorMap) * 4 * i, prepared[group[i]].maps, sizeof(CUtensorMap) * 4);
     std::vector<int> counts((size_t)max_k, 0), totals((size_t)max_k, 0);
     for (int it = 0; it < max_k; ++it) {
-      StepImage* images = reinterpret_cast<StepImage*>(host.data() + map_bytes + (size_t)it * (img_bytes + first_bytes));
-      int* first = reinterpret_cast<int*>(host.data() + map_bytes + (size_t)it * (img_bytes + first_bytes) + img_bytes);
+      StepImage* images = reinterpret_cast<StepImage*>(host.data() + (size_t)it * (img_bytes + first_bytes));
+      int* first = reinterpret_cast<int*>(host.data() + (size_t)it * (img_bytes + first_bytes) + img_bytes);
       int m = 0, items = 0;
       for (size_t i = 0; i < group.size(); ++i) {
         const CapturePlanes& cp = prepared[group[i]];
@@ -1991,12 +1875,9 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
         im.est_out = est[it & 1];
         im.W = job.W;
         im.H = job.H;
-        im.strips = (job.W + StepGeom<1>::QW - 2 * r - 1) / (StepGeom<1>::QW - 2 * r);
-        im.sg = cp.sg;
-        im.items = im.strips * cp.sg.segs;
-        // The first iteration reads the guide, later ones the estimate the one before wrote.
-        im.est_map = tma ? d_maps + 4 * i + (it == 0 ? 0 : 1 + ((it - 1) & 1)) : nullptr;
-        im.guide_map = tma ? d_maps + 4 * i + 3 : nullptr;
+        im.strips = strip_count(job.W, r);
+        im.segs = cp.segs;
+        im.items = im.strips * im.segs;
         first[m] = items;
         items += im.items;
         ++m;
@@ -2007,8 +1888,8 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
     }
     st = upload(ctx, tb, host.data(), table_bytes);
     for (int it = 0; it < max_k && st.ok(); ++it) {
-      const unsigned char* base = tb + map_bytes + (size_t)it * (img_bytes + first_bytes);
-      st = rl_step_images(ctx, r, tma, reinterpret_cast<const StepImage*>(base),
+      const unsigned char* base = tb + (size_t)it * (img_bytes + first_bytes);
+      st = rl_strip_images(ctx, r, vec, reinterpret_cast<const StepImage*>(base),
                           reinterpret_cast<const int*>(base + img_bytes), counts[(size_t)it], totals[(size_t)it],
                           prepared[g].taps);
     }
