@@ -130,6 +130,53 @@ RD_HD uint64_t chunk_breaks(const uint32_t* w, int count, uint32_t prev, bool se
   return m;
 }
 
+// Whether a run of three or more repeated bytes, the shortest that is sent as a
+// match, has a byte in the chunk (before and after: see chunk_tokens).
+RD_HD bool chunk_has_match(uint64_t breaks, int c0, int count, int before, int after) {
+  static_assert(CHUNK <= 32, "a chunk's repeats fit a word");
+  if (count == 0) return false;
+  const uint32_t rep = ~(uint32_t)breaks & (0xFFFFFFFFu >> (32 - count));
+  if (rep & (rep >> 1) & (rep >> 2)) return true;
+  // At most two repeats in a row: the runs at the chunk's ends may go on outside.
+  const int lead = (rep & 1u) + (uint32_t)((rep & 3u) == 3u);
+  const uint32_t top = rep << (32 - count);
+  const int tail = (int)(top >> 31) + (int)((top >> 30) == 3u);
+  const int left = c0 - 1 - before, right = after - (c0 + count);
+  return (lead > 0 && lead + left + (lead == count ? right : 0) >= 3) || (tail > 0 && tail + right >= 3);
+}
+
+RD_HD int ctz32(uint32_t v) {
+#if defined(__CUDA_ARCH__)
+  return __ffs((int)v) - 1;
+#else
+  return __builtin_ctz(v);
+#endif
+}
+
+// The chunk's tokens as bits: `literal` loses the bytes that matches cover,
+// `match` gets the first byte of each match that starts in the chunk
+// (run_token, a run at a time).
+RD_HD void chunk_matches(uint64_t breaks, int c0, int count, int before, int after, uint32_t& literal,
+                         uint32_t& match) {
+  uint32_t rest = ~(uint32_t)breaks & (0xFFFFFFFFu >> (32 - count));
+  while (rest) {
+    const int s = ctz32(rest);
+    const uint32_t from = rest >> s;  // ends in the run
+    const int len = from == 0xFFFFFFFFu ? 32 : ctz32(~from);
+    const int e = s + len;
+    rest &= e == 32 ? 0u : 0xFFFFFFFFu << e;
+    const int a = s == 0 ? before + 1 : c0 + s, b = e == count ? after : c0 + e;
+    if (b - a < 3) continue;
+    for (int p = a + (c0 + s - a) / MAX_RUN * MAX_RUN; p < c0 + e && b - p >= 3; p += MAX_RUN) {
+      // The match covers [p, min(p + MAX_RUN, b)).
+      const int lo = p < c0 + s ? s : p - c0;
+      const int hi = p + MAX_RUN < c0 + e ? p + MAX_RUN - c0 : e;
+      literal &= ~((0xFFFFFFFFu >> (32 - (hi - lo))) << lo);
+      if (p >= c0 + s) match |= 1u << lo;
+    }
+  }
+}
+
 // Calls visit(literal, 0) or visit(0, length) for each token that starts in
 // the chunk's first `count` bytes. `before` is the segment position of the
 // last break before the chunk (position 0 always is one) and `after` the
@@ -138,36 +185,37 @@ RD_HD uint64_t chunk_breaks(const uint32_t* w, int count, uint32_t prev, bool se
 template <class Visit>
 RD_HD void chunk_tokens(const uint32_t* w, uint64_t breaks, int c0, int count, int before, int after,
                         Visit&& visit) {
-  if (breaks == (1ull << count) - 1ull) {  // no byte repeats its predecessor: all literals
+  const uint32_t all = count == 0 ? 0u : 0xFFFFFFFFu >> (32 - count);
+  uint32_t literal = all, match = 0;
+  if (chunk_has_match(breaks, c0, count, before, after)) chunk_matches(breaks, c0, count, before, after, literal, match);
+  if (literal == 0xFFFFFFFFu) {  // a whole chunk of literals, the common case
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-    for (int j = 0; j < CHUNK; ++j) {
-      if (j >= count) break;
-      visit(chunk_byte(w, j), 0);
-    }
+    for (int j = 0; j < CHUNK; ++j) visit(chunk_byte(w, j), 0);
     return;
   }
+  // The rare case word by word, the words moving up: a small loop, so that the
+  // common case stays in the instruction cache.
+  uint32_t t[CHUNK_WORDS];
+  for (int k = 0; k < CHUNK_WORDS; ++k) t[k] = w[k];
 #if defined(__CUDA_ARCH__)
-#pragma unroll
+#pragma unroll 1
 #endif
-  for (int j = 0; j < CHUNK; ++j) {
-    if (j >= count) break;
-    const uint32_t x = chunk_byte(w, j);
-    if ((breaks >> j) & 1ull) {
-      visit(x, 0);
-      continue;
+  for (int j0 = 0; j0 < count; j0 += 4) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int j = j0; j < j0 + 4; ++j) {
+      if ((literal >> j) & 1u) {
+        visit((t[0] >> (8 * (j & 3))) & 0xFFu, 0);
+      } else if ((match >> j) & 1u) {
+        const uint32_t above = j == CHUNK - 1 ? 0u : (uint32_t)breaks & (0xFFFFFFFEu << j);
+        const int b = above ? c0 + ctz32(above) : after;
+        visit(0u, b - (c0 + j) < MAX_RUN ? b - (c0 + j) : MAX_RUN);
+      }
     }
-    const uint64_t upto = j == CHUNK - 1 ? ~0ull : (2ull << j) - 1ull;
-    const uint64_t below = breaks & upto;
-    const uint64_t above = breaks & ~upto;
-    const int a = (below ? c0 + 63 - clz64(below) : before) + 1;
-    const int b = above ? c0 + ctz64(above) : after;
-    const int t = run_token(c0 + j, a, b);
-    if (t == 1)
-      visit(x, 0);
-    else if (t >= 3)
-      visit(0u, t);
+    for (int k = 0; k + 1 < CHUNK_WORDS; ++k) t[k] = t[k + 1];
   }
 }
 
