@@ -1,6 +1,7 @@
 // The C ABI (include/rd_gpu.h): context, processor API, stage entry points and
 // host contract helpers. Everything device-side is ordered on the context's
-// stream; device memory comes from the stream-ordered pool (cudaMallocAsync)
+// stream; device memory comes from the stream-ordered pool (cudaMallocAsync),
+// in blocks that the context keeps from call to call,
 // and is charged against the context's byte budget before it is taken, like
 // the reference's logical reservations (crates/gpu/src/memory.rs:44-60).
 #include <cuda_runtime.h>
@@ -32,22 +33,126 @@ Status reserve(Context& ctx, size_t bytes) {
 }
 void release(Context& ctx, size_t bytes) { ctx.reserved -= std::min<uint64_t>(bytes, ctx.reserved); }
 
+// Every context's kept blocks can be given back when the device runs out of
+// memory; the registry is what finds them.
+std::mutex g_contexts_mutex;
+std::vector<Context*> g_contexts;
+
+void release_kept_blocks(Context& ctx) {
+  std::lock_guard<std::mutex> lk(ctx.blocks.mutex);
+  for (auto& b : ctx.blocks.kept) cudaFreeAsync(b.first, ctx.stream);
+  ctx.blocks.kept.clear();
+  ctx.blocks.bytes = 0;
+}
+
+// Pinning memory takes longer than a batch's whole set-up, and a batch makes its
+// contexts anew: up to eight areas (528 KB each) wait here for the next context.
+constexpr size_t SPARE_AREAS = 8;
+std::vector<unsigned char*> g_spare_areas;  // under g_contexts_mutex
+
+bool take_pinned_area(PinnedArea& a) {
+  constexpr size_t bytes = 2 * PinnedArea::HALF + PinnedArea::READBACK;
+  for (auto& e : a.done)
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) e = nullptr;
+  if (a.done[0] && a.done[1]) {
+    std::lock_guard<std::mutex> lk(g_contexts_mutex);
+    if (!g_spare_areas.empty()) {
+      a.base = g_spare_areas.back();
+      g_spare_areas.pop_back();
+      a.pinned = true;
+    }
+  }
+  if (!a.base && a.done[0] && a.done[1]) {
+    void* p = nullptr;
+    a.pinned = cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess;
+    if (a.pinned) a.base = static_cast<unsigned char*>(p);
+  }
+  cudaGetLastError();
+  if (!a.base) a.base = new (std::nothrow) unsigned char[bytes];
+  return a.base != nullptr;
+}
+// After the last copy into or out of it.
+void give_pinned_area(PinnedArea& a) {
+  if (a.pinned) {
+    std::lock_guard<std::mutex> lk(g_contexts_mutex);
+    if (g_spare_areas.size() < SPARE_AREAS) g_spare_areas.push_back(a.base);
+    else cudaFreeHost(a.base);
+  } else {
+    delete[] a.base;
+  }
+  for (auto& e : a.done)
+    if (e) cudaEventDestroy(e);
+}
+
+// Memory comes from the stream-ordered pool, through the context's kept blocks.
+// The pool maps memory anew where no freed block of its own fits, 80 to 90 us
+// each for the large planes of a 24 MP develop while the GPU waits; a call's
+// blocks have the sizes of the last call's, so the next takes them as they are.
+// A kept block is reused in the order of the context's stream, like one that
+// the pool hands out again. Under stream capture the pool is asked directly.
 Status device_alloc(Context& ctx, size_t bytes, void** out) {
   *out = nullptr;
   if (bytes == 0) bytes = 16;
   RD_TRY(reserve(ctx, bytes));
-  const cudaError_t e = cudaMallocAsync(out, bytes, ctx.stream);
+  BlockCache& cache = ctx.blocks;
+  if (!ctx.capturing) {
+    std::lock_guard<std::mutex> lk(cache.mutex);
+    for (size_t k = cache.kept.size(); k-- > 0;)
+      if (cache.kept[k].second == bytes) {
+        *out = cache.kept[k].first;
+        cache.kept.erase(cache.kept.begin() + (long)k);
+        cache.bytes -= bytes;
+        cache.live[*out] = bytes;
+        return Status{};
+      }
+  }
+  cudaError_t e = cudaMallocAsync(out, bytes, ctx.stream);
+  if (e != cudaSuccess && !ctx.capturing) {
+    cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> lk(g_contexts_mutex);
+      for (Context* c : g_contexts)
+        if (c->device == ctx.device && !c->capturing) {
+          release_kept_blocks(*c);
+          cudaStreamSynchronize(c->stream);
+        }
+    }
+    e = cudaMallocAsync(out, bytes, ctx.stream);
+  }
   if (e != cudaSuccess) {
     release(ctx, bytes);
     cudaGetLastError();
     return Status{RD_OVER_BUDGET, std::string("device allocation failed: ") + cudaGetErrorString(e)};
   }
+  if (!ctx.capturing) {
+    std::lock_guard<std::mutex> lk(cache.mutex);
+    cache.live[*out] = bytes;
+  }
   return Status{};
 }
 void device_free(Context& ctx, void* ptr, size_t bytes) {
   if (!ptr) return;
-  cudaFreeAsync(ptr, ctx.stream);
   release(ctx, bytes == 0 ? 16 : bytes);
+  {
+    BlockCache& cache = ctx.blocks;
+    std::lock_guard<std::mutex> lk(cache.mutex);
+    const auto it = cache.live.find(ptr);
+    if (it != cache.live.end()) {
+      const size_t size = it->second;
+      cache.live.erase(it);
+      if (!ctx.capturing && size <= BLOCK_CACHE_BYTES) {
+        cache.kept.emplace_back(ptr, size);
+        cache.bytes += size;
+        while (cache.bytes > BLOCK_CACHE_BYTES || cache.kept.size() > BLOCK_CACHE_BLOCKS) {
+          cudaFreeAsync(cache.kept.front().first, ctx.stream);
+          cache.bytes -= cache.kept.front().second;
+          cache.kept.erase(cache.kept.begin());
+        }
+        return;
+      }
+    }
+  }
+  cudaFreeAsync(ptr, ctx.stream);
 }
 
 const char* kernel_family_name(int family) {
@@ -109,8 +214,36 @@ Status set_stream_priority(Context& c, bool high) {
   return Status{};
 }
 
+// Host data to the device; `src` may change once this returns. Small uploads go
+// through the pinned area: a copy out of pageable memory makes the host wait for
+// the stream from 64 KB on (the area reduction's tables for the whole remap
+// before it), and for the driver's own staging below.
 Status upload(Context& ctx, void* dst, const void* src, size_t bytes) {
   if (!ctx.capturing) {
+    PinnedArea& area = ctx.pinned;
+    if (area.pinned && bytes <= PinnedArea::HALF) {
+      std::lock_guard<std::mutex> lk(ctx.blocks.mutex);
+      bool room = area.used + bytes <= PinnedArea::HALF;
+      if (!room) {
+        const int other = area.half ^ 1;
+        RD_CUDA_TRY(cudaEventRecord(area.done[area.half], ctx.stream));
+        area.filled[area.half] = true;
+        if (!area.filled[other] || cudaEventQuery(area.done[other]) == cudaSuccess) {
+          area.half = other;
+          area.used = 0;
+          room = true;
+        } else {
+          cudaGetLastError();  // not ready: this one goes the other way
+        }
+      }
+      if (room) {
+        unsigned char* at = area.base + (size_t)area.half * PinnedArea::HALF + area.used;
+        std::memcpy(at, src, bytes);
+        area.used += (bytes + 63) & ~(size_t)63;
+        RD_CUDA_TRY(cudaMemcpyAsync(dst, at, bytes, cudaMemcpyHostToDevice, ctx.stream));
+        return Status{};
+      }
+    }
     RD_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx.stream));
     return Status{};
   }
@@ -124,9 +257,11 @@ Status upload(Context& ctx, void* dst, const void* src, size_t bytes) {
 
 Status check_kernel_error(Context& ctx, const char* stage) {
   if (ctx.capturing) return Status{};  // read after the graph has run
-  uint32_t word = 0;
-  RD_CUDA_TRY(cudaMemcpyAsync(&word, ctx.d_error, sizeof(word), cudaMemcpyDeviceToHost, ctx.stream));
+  RD_CUDA_TRY(cudaMemcpyAsync(readback(ctx, READBACK_ERROR), ctx.d_error, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                              ctx.stream));
   RD_CUDA_TRY(cudaStreamSynchronize(ctx.stream));
+  uint32_t word = 0;
+  std::memcpy(&word, readback(ctx, READBACK_ERROR), sizeof(word));
   if (!ctx.pending.empty()) resolve_kernel_timing(ctx);
   if (!ctx.tune_runs.empty()) resolve_rl_tuning(ctx);
   if (!ctx.shape_runs.empty()) resolve_shape_tuning(ctx);
@@ -498,7 +633,8 @@ Status develop_impl(rd_ctx* h, const uint16_t* d_raw, size_t row_stride, const r
   if (d_mosaic) rd::device_free(ctx, d_mosaic, mosaic_bytes);
   uint64_t host_stats[16] = {};
   if (st.ok() && !ctx.capturing) {
-    const cudaError_t e = cudaMemcpyAsync(host_stats, d_stats, sizeof(host_stats), cudaMemcpyDeviceToHost, ctx.stream);
+    const cudaError_t e = cudaMemcpyAsync(rd::readback(ctx, rd::READBACK_STATS), d_stats, sizeof(host_stats),
+                                          cudaMemcpyDeviceToHost, ctx.stream);
     if (e != cudaSuccess) st = Status{RD_READBACK, cudaGetErrorString(e)};
   }
   rd::device_free(ctx, d_stats, sizeof(unsigned long long) * 16);
@@ -512,6 +648,7 @@ Status develop_impl(rd_ctx* h, const uint16_t* d_raw, size_t row_stride, const r
     cudaStreamSynchronize(ctx.stream);
     return st;
   }
+  if (!ctx.capturing) std::memcpy(host_stats, rd::readback(ctx, rd::READBACK_STATS), sizeof(host_stats));
   if (metrics) {
     metrics->normalize_highlight_ms = tm.span(0, 1);
     metrics->demosaic_ms = tm.span(1, 2);
@@ -576,6 +713,12 @@ rd_status rd_ctx_create(int device, uint64_t budget_bytes, rd_ctx** out) {
     return RD_SYNCHRONIZATION;
   }
   c.d_work = c.d_error + 1;
+  if (!rd::take_pinned_area(c.pinned)) {
+    cudaFree(c.d_error);
+    cudaStreamDestroy(c.stream);
+    delete h;
+    return RD_OVER_BUDGET;
+  }
   // Keep freed pool memory cached between calls instead of returning it to the driver.
   cudaMemPool_t pool;
   if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
@@ -583,6 +726,10 @@ rd_status rd_ctx_create(int device, uint64_t budget_bytes, rd_ctx** out) {
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
   }
   cudaStreamSynchronize(c.stream);
+  {
+    std::lock_guard<std::mutex> lk(rd::g_contexts_mutex);
+    rd::g_contexts.push_back(&c);
+  }
   *out = h;
   return RD_OK;
 }
@@ -594,8 +741,14 @@ void rd_ctx_destroy(rd_ctx* h) {
   cudaSetDevice(c.device);
   if (c.amaze_scratch) rd::device_free(c, c.amaze_scratch, c.amaze_bytes);
   if (c.flush_buf) rd::device_free(c, c.flush_buf, c.flush_bytes);
+  {
+    std::lock_guard<std::mutex> lk(rd::g_contexts_mutex);
+    rd::g_contexts.erase(std::find(rd::g_contexts.begin(), rd::g_contexts.end(), &c));
+  }
+  rd::release_kept_blocks(c);
   cudaStreamSynchronize(c.stream);
   for (void* p : c.pinned_uploads) cudaFreeHost(p);
+  rd::give_pinned_area(c.pinned);
   rd::resolve_kernel_timing(c);
   for (auto& r : c.tune_runs) {
     cudaEventDestroy(r.second.first);
@@ -812,17 +965,18 @@ rd_status rd_render(rd_ctx* h, const rd_base* cbase, const rd_color_desc* color,
       cs = Status{RD_READBACK, "histogram readback failed"};
     return finish(h, cs);
   }
-  uint64_t bins[1024];
+  uint64_t* bins = static_cast<uint64_t*>(rd::readback(ctx, rd::READBACK_BINS));
+  const size_t bins_bytes = 1024 * sizeof(uint64_t);
   Status st;
   if (srgb_out &&
       cudaMemcpyAsync(srgb_out, base->d_srgb, (size_t)3 * base->W * base->H, cudaMemcpyDeviceToHost, ctx.stream) !=
           cudaSuccess)
     st = Status{RD_READBACK, "output readback failed"};
-  if (st.ok() && cudaMemcpyAsync(bins, base->d_hist, sizeof(bins), cudaMemcpyDeviceToHost, ctx.stream) != cudaSuccess)
+  if (st.ok() && cudaMemcpyAsync(bins, base->d_hist, bins_bytes, cudaMemcpyDeviceToHost, ctx.stream) != cudaSuccess)
     st = Status{RD_READBACK, "histogram readback failed"};
   if (st.ok() && cudaStreamSynchronize(ctx.stream) != cudaSuccess) st = Status{RD_READBACK, "readback failed"};
   if (st.ok()) {
-    if (hist) std::memcpy(hist, bins, sizeof(bins));
+    if (hist) std::memcpy(hist, bins, bins_bytes);
     // Histogram::count_clipped (histogram.rs:110-121): bins 0 and 255.
     if (clipped)
       for (int c = 0; c < 3; ++c) {

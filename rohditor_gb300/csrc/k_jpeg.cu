@@ -457,7 +457,8 @@ Status run_jpeg_encode(Context& ctx, const uint8_t* d_rgb, int W, int H, int qua
   for (int k = 0; k < 64; ++k) cp.zigzag_of[zz[k]] = (uint8_t)k;
 
   Status st;
-  uint32_t h_hist[TABLES * 256];
+  const uint32_t* h_hist = static_cast<const uint32_t*>(readback(ctx, READBACK_BINS));
+  static_assert(READBACK_BINS + TABLES * 256 * sizeof(uint32_t) <= PinnedArea::READBACK, "the counts fit the area");
   if (cudaMemsetAsync(hist, 0, TABLES * 256 * 4, ctx.stream) != cudaSuccess)
     st = Status{RD_SYNCHRONIZATION, "histogram clear failed"};
   if (st.ok()) {
@@ -467,7 +468,8 @@ Status run_jpeg_encode(Context& ctx, const uint8_t* d_rgb, int W, int H, int qua
     RD_LAUNCH(ctx, K_ENCODE,
               jpeg_hist_kernel<<<(unsigned)((blocks * 3 + HIST_THREADS - 1) / HIST_THREADS), HIST_THREADS, 0,
                                  ctx.stream>>>(coef, blocks, hist));
-    if (cudaMemcpyAsync(h_hist, hist, sizeof(h_hist), cudaMemcpyDeviceToHost, ctx.stream) != cudaSuccess ||
+    if (cudaMemcpyAsync(readback(ctx, READBACK_BINS), hist, TABLES * 256 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                        ctx.stream) != cudaSuccess ||
         cudaStreamSynchronize(ctx.stream) != cudaSuccess)
       st = Status{RD_SYNCHRONIZATION, "JPEG symbol counts readback failed"};
   }

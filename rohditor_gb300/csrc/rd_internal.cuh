@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -63,6 +64,29 @@ struct ShapePick {
   int value = 0;
   cudaEvent_t start = nullptr;  // set when this launch is timed
 };
+// Device blocks that a context has freed and keeps for its next allocation of
+// the same size, oldest first, and the sizes of those it has handed out.
+struct BlockCache {
+  std::mutex mutex;
+  std::vector<std::pair<void*, size_t>> kept;
+  std::unordered_map<void*, size_t> live;
+  size_t bytes = 0;  // of the kept blocks
+};
+constexpr size_t BLOCK_CACHE_BYTES = size_t(8) << 30;
+constexpr size_t BLOCK_CACHE_BLOCKS = 64;
+
+// Pinned host memory of a context: two halves that small uploads go through in
+// turn, and a place for what a call reads back.
+struct PinnedArea {
+  static constexpr size_t HALF = 256 << 10, READBACK = 16 << 10;
+  unsigned char* base = nullptr;  // HALF, HALF, READBACK; pageable (and no staging) where pinning failed
+  bool pinned = false;
+  size_t used = 0;                // of the current half
+  int half = 0;
+  bool filled[2] = {false, false};
+  cudaEvent_t done[2] = {};       // after the last copy out of each half
+};
+
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -103,6 +127,8 @@ struct Context {
   // one item.
   bool yield_sms = false;
   std::vector<void*> pinned_uploads;
+  BlockCache blocks;
+  PinnedArea pinned;
   // Timed RL iterations of a launch-shape tuning run, resolved after the
   // stage's synchronisation: (candidate segment count, start, end).
   int tune_shape[3] = {0, 0, 0};
@@ -119,6 +145,10 @@ struct Context {
   uint32_t wait_limit = 0;      // 0: the built-in limits
   int32_t wait_withhold = 0;    // RD_WAIT_* of include/rd_gpu.h
 };
+
+// Places in the readback area (each used and read within one call).
+constexpr size_t READBACK_ERROR = 0, READBACK_STATS = 64, READBACK_BINS = 1024;
+inline void* readback(Context& ctx, size_t at) { return ctx.pinned.base + 2 * PinnedArea::HALF + at; }
 
 // Iteration limits of the device waits when no test sets one.
 constexpr uint32_t AMAZE_DEFAULT_WAIT_TRIES = 1u << 22;
