@@ -348,7 +348,24 @@ static MosaicSource make_source(const rd_sensor_desc& s, const uint16_t* d_raw, 
     m.black[k] = s.black[k];
     m.white[k] = s.white[k];
   }
+  set_parity_levels(m);
   return m;
+}
+
+void set_parity_levels(MosaicSource& m) {
+  m.parity_levels = m.black_w <= 2 && m.black_h <= 2;
+  for (int k = 0; k < 4 && m.parity_levels; ++k) {
+    const int sx = m.crop_x + (k & 1), sy = m.crop_y + (k >> 1);
+    const int bi = (sy % m.black_h) * m.black_w + sx % m.black_w;
+    const float black = m.black[bi];
+    const float white =
+        m.white_count == 1 ? m.white[0] : m.white[m.white_count == 3 ? color_at(m.sensor_cfa, sx, sy) : bi];
+    const float span = white - black, size = std::fabs(black);
+    m.level_black[k] = black;
+    m.level_span[k] = span;
+    if (!((black == 0.0f || size >= 0x1p-60f) && size <= 0x1p30f && span >= 0x1p-30f && span <= 0x1p30f))
+      m.parity_levels = 0;
+  }
 }
 
 // build_plan (crates/optics/src/plan.rs:173-231) and find_scale (:521-559).

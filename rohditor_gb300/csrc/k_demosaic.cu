@@ -23,13 +23,14 @@ namespace {
 
 // Warp-aggregated Clip statistics of one pixel: affected, changed, over white, affected per channel.
 struct ClipTally {
-  unsigned long long v[6] = {0, 0, 0, 0, 0, 0};
+  unsigned v[6] = {0, 0, 0, 0, 0, 0};
   __device__ void add(const MosaicSource& s, int x, int y) {
     const int ch = color_at(s.cfa, x, y);
     add_value(source_normalized(s, x, y), ch, s.clip_levels[ch]);
   }
   // One normalized sample of channel ch against its Clip ceiling.
-  __device__ void add_value(float value, int ch, float limit) {
+  __device__ __forceinline__ void add_value(float value, int ch, float limit) {
+    if (!(value >= limit || value > 1.0f)) return;
     if (value >= limit) {
       v[0]++;
       // Constant indexes keep the counters in registers.
@@ -42,9 +43,8 @@ struct ClipTally {
   }
   __device__ void flush(unsigned long long* out) {
     for (int c = 0; c < 6; ++c) {
-      unsigned long long s = v[c];
-      for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-      if ((threadIdx.x & 31) == 0 && s) atomicAdd(&out[c], s);
+      const unsigned s = __reduce_add_sync(0xffffffffu, v[c]);
+      if ((threadIdx.x & 31) == 0 && s) atomicAdd(&out[c], (unsigned long long)s);
     }
   }
 };
@@ -208,7 +208,35 @@ __global__ void __launch_bounds__(256) quad_kernel(const MosaicSource src, int m
       }
       return;
     }
-    if (load == QUAD_TMA_U16 || convert) {
+    if (load == QUAD_TMA_U16 && src.parity_levels) {
+      // By 2x2 cells: levels, colour and ceiling of each position are the same
+      // in every cell. Sample by sample, with level look-ups and an IEEE
+      // division each, the tile's conversion was two thirds of the kernel: a
+      // 45 MP frame took 0.33 ms, 0.20 now (its bytes take 0.095).
+      float span_y[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) span_y[j] = reciprocal_of(src.level_span[j]);
+      constexpr int CW = QFW / 2;
+      for (int k = tid; k < QFH / 2 * CW; k += 256) {
+        const int r = 2 * (k / CW), c = 2 * (k % CW);
+        const int x = x0 - 4 + c, y = y0 - 2 + r;
+        const unsigned top = *reinterpret_cast<const unsigned*>(&S.raw[r][c + 4]);
+        const unsigned low = *reinterpret_cast<const unsigned*>(&S.raw[r + 1][c + 4]);
+        const unsigned raw[4] = {top & 0xffffu, top >> 16, low & 0xffffu, low >> 16};
+        const bool core = count_clip && r >= 2 && r < QH + 2 && c >= 4 && c < QW + 4;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          constexpr int COLOR[4] = {cfa_color(CFA, 0, 0), cfa_color(CFA, 1, 0), cfa_color(CFA, 0, 1), cfa_color(CFA, 1, 1)};
+          const bool inside = (unsigned)(x + (j & 1)) < (unsigned)W && (unsigned)(y + (j >> 1)) < (unsigned)H;
+          const float n = normalize_parity(src, raw[j], j, span_y[j]);
+          v[j] = inside ? staged_value(src, n, COLOR[j]) : 0.0f;
+          if (core && inside) tally_value(tally, src, n, COLOR[j]);
+        }
+        *reinterpret_cast<float2*>(&S.t[r][c]) = make_float2(v[0], v[1]);
+        *reinterpret_cast<float2*>(&S.t[r + 1][c]) = make_float2(v[2], v[3]);
+      }
+    } else if (load == QUAD_TMA_U16 || convert) {
       for (int k = tid; k < QFH * QFW; k += 256) {
         const int r = k / QFW, c = k % QFW;
         const int x = x0 - 4 + c, y = y0 - 2 + r;
@@ -381,12 +409,21 @@ __device__ __forceinline__ float nonzero(float v) {
   if (fabsf(v) >= REPS) return v;
   return signbit(v) ? -REPS : REPS;
 }
-__device__ __forceinline__ float ratio_estimate(float sample, float lp, float nlp) {
-  const float d = nonzero(REPS + lp + nlp);
-  return sample * (2.0f * lp) / d;
-}
-__device__ __forceinline__ float weighted_pair(float w1, float v1, float w2, float v2) {
-  return (w1 * v1 + w2 * v2) / nonzero(w1 + w2);
+// N quotients. QUICK: every sample of the window is of a magnitude up to 2^20, so
+// divisors (1e-10 or more) and numerators stay in quick_div's range but for
+// numerators next to zero, which are looked for once for all N.
+template <bool QUICK, int N>
+__device__ __forceinline__ void rcd_quotients(const float (&a)[N], const float (&b)[N], float (&q)[N]) {
+  float least = 1.0f;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    q[k] = QUICK ? quick_div(a[k], b[k]) : a[k] / b[k];
+    least = fminf(least, fabsf(a[k]));
+  }
+  if (QUICK && least < 7.8886091e-31f) {  // 2^-100
+#pragma unroll
+    for (int k = 0; k < N; ++k) q[k] = a[k] / b[k];
+  }
 }
 __device__ __forceinline__ float refined_direction(float c, float nw, float ne, float sw, float se) {
   const float n = 0.25f * (nw + ne + sw + se);
@@ -409,6 +446,187 @@ __device__ __forceinline__ float rmaxf(float a, float b) {
   return a > b ? a : b;
 }
 
+// Each of `rows` rows of SITES sites once: f(row, site), the block's threads
+// walking the sites row after row. A step advances by a constant number of rows
+// and sites; a division and a remainder for each site, and looking its colour up
+// in the pattern, were an eighth of the kernel's instructions.
+template <int SITES, class F>
+__device__ __forceinline__ void for_sites(int rows, F&& f) {
+  constexpr int DROW = RTHREADS / SITES, DSITE = RTHREADS % SITES;
+  int row = (int)threadIdx.x / SITES, site = (int)threadIdx.x % SITES;
+  while (row < rows) {
+    f(row, site);
+    row += DROW;
+    site += DSITE;
+    if (site >= SITES) {
+      site -= SITES;
+      ++row;
+    }
+  }
+}
+
+// The same over sites in every other column whose parity changes from row to
+// row (red/blue or green ones): consecutive threads take the sites of two rows in
+// turn. A row's sites share the parity of their banks, two rows' cover both, so
+// a warp's loads do not collide: with a row at a time each took two passes.
+// Shared memory bounds the kernel; a 12 MP frame took 0.456 ms with a row at a
+// time and IEEE divisions, 0.426 now.
+template <int SITES, class F>
+__device__ __forceinline__ void for_checkered_sites(int rows, F&& f) {
+  for_sites<2 * SITES>(rows / 2, [&](int pair, int t) { f(2 * pair + (t & 1), t >> 1); });
+}
+
+// The stages between the samples and the window's three colours (their planes
+// and scratch: RcdSmem).
+template <bool QUICK>
+__device__ void rcd_stages(RcdSmem& S, int tp) {
+  float* const cfa = S.cfa + 2;
+  float* const R0 = S.rgb[0] + 2;
+  float* const G1 = S.rgb[1] + 2;
+  float* const B2 = S.rgb[2] + 2;
+  float* const vh = S.vh + 2;
+  float* const vhp = S.hp[0] + 2;
+  float* const hhp = S.hp[1] + 2;
+  float* const pcd = S.hp[0];  // half planes (index / 2)
+  float* const qcd = S.hp[1];
+  float* const pq = S.pq;
+  // Columns of the red/blue sites: even in rows of this parity, else odd; the other way round for green.
+  const int odd0 = color_at(tp, 0, 0) & 1;
+  const bool red0 = color_at(tp, odd0, 0) == 0;  // row 0 holds red (else blue)
+  // ---- squared high passes (rcd_stages.rs:8-48, 393-404): vertical at rows
+  //      [3, RW-3) x cols [4, RW-4), horizontal at rows [4, RW-4) x cols [3, RW-3)
+  for_sites<RW - 6>(RW - 6, [&](int row, int col) {
+    const int r = 3 + row, c = 3 + col;
+    const int i = r * RP + c;
+    if (c >= 4 && c < RW - 4)
+      vhp[i] = rsq((cfa[i - 3 * RP] - cfa[i - RP] - cfa[i + RP] + cfa[i + 3 * RP]) -
+                   3.0f * (cfa[i - 2 * RP] + cfa[i + 2 * RP]) + 6.0f * cfa[i]);
+    if (r >= 4 && r < RW - 4)
+      hhp[i] = rsq((cfa[i - 3] - cfa[i - 1] - cfa[i + 1] + cfa[i + 3]) - 3.0f * (cfa[i - 2] + cfa[i + 2]) + 6.0f * cfa[i]);
+  });
+  __syncthreads();
+  // ---- find_directions (rcd_stages.rs:8-48) at [4, RW-4)^2 and the low pass
+  //      (:55-82) at the red/blue sites of [2, RW-2)^2
+  for_sites<RW - 8>(RW - 8, [&](int row, int col) {
+    const int r = 4 + row, c = 4 + col;
+    const int i = r * RP + c;
+    const float vs = rmaxf(vhp[i - RP] + vhp[i] + vhp[i + RP], REPS2);
+    const float hs = rmaxf(hhp[i - 1] + hhp[i] + hhp[i + 1], REPS2);
+    vh[i] = QUICK ? quick_div(vs, vs + hs) : vs / (vs + hs);
+  });
+  for_checkered_sites<(RW - 4) / 2>(RW - 4, [&](int row, int site) {
+    const int r = 2 + row;
+    const int c = 2 + (odd0 ^ (r & 1)) + 2 * site;
+    const int i = r * RP + c;
+    pq[i / 2] = cfa[i] + 0.5f * (cfa[i - RP] + cfa[i + RP] + cfa[i - 1] + cfa[i + 1]) +
+                0.25f * (cfa[i - RP - 1] + cfa[i - RP + 1] + cfa[i + RP - 1] + cfa[i + RP + 1]);
+  });
+  __syncthreads();
+  // ---- interpolate_green (rcd_stages.rs:84-147) at the red/blue sites of
+  //      [4, RW-4)^2; calculate_diagonal_high_pass (:162-196) at the odd
+  //      columns of [3, RW-3)^2 (into the high-pass area, now free)
+  static_assert(RW % 2 == 0, "rows pair up");
+  constexpr int SITES4 = (RW - 8) / 2;  // red/blue sites per row of [4, RW-4)
+  for_checkered_sites<SITES4>(RW - 8, [&](int row, int site) {
+    const int r = 4 + row;
+    const int c = 4 + (odd0 ^ (r & 1)) + 2 * site;
+    const int i = r * RP + c;
+    const float ng = cardinal_gradient(cfa, i, -RP), sg = cardinal_gradient(cfa, i, RP);
+    const float wg = cardinal_gradient(cfa, i, -1), eg = cardinal_gradient(cfa, i, 1);
+    const int li = i / 2;
+    const float lp = pq[li];
+    // The four ratio estimates sample * 2 lp / (lp + its neighbour's), then the
+    // gradients' weighted means of opposite ones.
+    const float lp2 = 2.0f * lp;
+    const float num[4] = {cfa[i - RP] * lp2, cfa[i + RP] * lp2, cfa[i - 1] * lp2, cfa[i + 1] * lp2};
+    const float den[4] = {nonzero(REPS + lp + pq[li - RP]), nonzero(REPS + lp + pq[li + RP]),
+                          nonzero(REPS + lp + pq[li - 1]), nonzero(REPS + lp + pq[li + 1])};
+    float est[4], mean[2];  // north, south, west, east
+    rcd_quotients<QUICK>(num, den, est);
+    const float wsum[2] = {sg * est[0] + ng * est[1], wg * est[3] + eg * est[2]};
+    const float weight[2] = {nonzero(sg + ng), nonzero(wg + eg)};
+    rcd_quotients<QUICK>(wsum, weight, mean);
+    const float ve = mean[0], he = mean[1];
+    const float dir = refined_direction(vh[i], vh[i - RP - 1], vh[i - RP + 1], vh[i + RP - 1], vh[i + RP + 1]);
+    G1[i] = interpolate(dir, he, ve);
+  });
+  constexpr int ODD3 = (RW - 6) / 2;  // odd columns of [3, RW-3)
+  for_sites<ODD3>(RW - 6, [&](int row, int site) {
+    const int r = 3 + row, c = 3 + 2 * site;
+    const int i = r * RP + c;
+    pcd[i / 2] = rsq((cfa[i - 3 * RP - 3] - cfa[i - RP - 1] - cfa[i + RP + 1] + cfa[i + 3 * RP + 3]) -
+                     3.0f * (cfa[i - 2 * RP - 2] + cfa[i + 2 * RP + 2]) + 6.0f * cfa[i]);
+    qcd[i / 2] = rsq((cfa[i - 3 * RP + 3] - cfa[i - RP + 1] - cfa[i + RP - 1] + cfa[i + 3 * RP - 3]) -
+                     3.0f * (cfa[i - 2 * RP + 2] + cfa[i + 2 * RP - 2]) + 6.0f * cfa[i]);
+  });
+  __syncthreads();
+  // ---- calculate_diagonal_directions (rcd_stages.rs:198-225), into pq
+  for_checkered_sites<SITES4>(RW - 8, [&](int row, int site) {
+    const int r = 4 + row;
+    const int c = 4 + (odd0 ^ (r & 1)) + 2 * site;
+    const int i = r * RP + c;
+    const int hi = i / 2, pr = (i - RP - 1) / 2, nr = (i + RP - 1) / 2;
+    const float ps = rmaxf(pcd[pr] + pcd[hi] + pcd[nr + 1], REPS2);
+    const float qs = rmaxf(qcd[pr + 1] + qcd[hi] + qcd[nr], REPS2);
+    pq[hi] = QUICK ? quick_div(ps, ps + qs) : ps / (ps + qs);
+  });
+  __syncthreads();
+  // ---- interpolate_opposite_color (rcd_stages.rs:227-285)
+  for_checkered_sites<SITES4>(RW - 8, [&](int row, int site) {
+    const int r = 4 + row;
+    const int c = 4 + (odd0 ^ (r & 1)) + 2 * site;
+    const int i = r * RP + c;
+    const int hi = i / 2, pr = (i - RP - 1) / 2, nr = (i + RP - 1) / 2;
+    const float dir = refined_direction(pq[hi], pq[pr], pq[pr + 1], pq[nr], pq[nr + 1]);
+    float* const v = red0 == ((r & 1) == 0) ? B2 : R0;  // the row's missing colour
+    const float* g = G1;
+    const float nwg = diagonal_gradient(v, g, i, -RP - 1), neg = diagonal_gradient(v, g, i, -RP + 1);
+    const float swg = diagonal_gradient(v, g, i, RP - 1), seg = diagonal_gradient(v, g, i, RP + 1);
+    const float nwe = v[i - RP - 1] - g[i - RP - 1], nee = v[i - RP + 1] - g[i - RP + 1];
+    const float swe = v[i + RP - 1] - g[i + RP - 1], see = v[i + RP + 1] - g[i + RP + 1];
+    const float wsum[2] = {nwg * see + seg * nwe, neg * swe + swg * nee};
+    const float weight[2] = {nonzero(nwg + seg), nonzero(neg + swg)};
+    float mean[2];
+    rcd_quotients<QUICK>(wsum, weight, mean);
+    v[i] = g[i] + interpolate(dir, mean[1], mean[0]);
+  });
+  __syncthreads();
+  // ---- interpolate_at_green (rcd_stages.rs:287-355) at the green sites of [4, RW-4)^2
+  for_checkered_sites<SITES4>(RW - 8, [&](int row, int site) {
+    const int r = 4 + row;
+    const int c = 4 + (odd0 ^ (r & 1) ^ 1) + 2 * site;
+    const int i = r * RP + c;
+    const float dir = refined_direction(vh[i], vh[i - RP - 1], vh[i - RP + 1], vh[i + RP - 1], vh[i + RP + 1]);
+    const float* g = G1;
+    const float green = g[i];
+    const float n1 = REPS + fabsf(green - g[i - 2 * RP]);
+    const float s1 = REPS + fabsf(green - g[i + 2 * RP]);
+    const float w1 = REPS + fabsf(green - g[i - 2]);
+    const float e1 = REPS + fabsf(green - g[i + 2]);
+    const float gn = g[i - RP], gs = g[i + RP], gw = g[i - 1], ge = g[i + 1];
+    float wsum[4], weight[4], mean[4];  // vertical and horizontal of red, of blue
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float* v = k == 0 ? R0 : B2;
+      const float nsa = fabsf(v[i - RP] - v[i + RP]);
+      const float ewa = fabsf(v[i - 1] - v[i + 1]);
+      const float ngr = n1 + nsa + fabsf(v[i - RP] - v[i - 3 * RP]);
+      const float sgr = s1 + nsa + fabsf(v[i + RP] - v[i + 3 * RP]);
+      const float wgr = w1 + ewa + fabsf(v[i - 1] - v[i - 3]);
+      const float egr = e1 + ewa + fabsf(v[i + 1] - v[i + 3]);
+      const float ne = v[i - RP] - gn, se = v[i + RP] - gs, we = v[i - 1] - gw, ee = v[i + 1] - ge;
+      wsum[2 * k] = ngr * se + sgr * ne;
+      weight[2 * k] = nonzero(ngr + sgr);
+      wsum[2 * k + 1] = egr * we + wgr * ee;
+      weight[2 * k + 1] = nonzero(egr + wgr);
+    }
+    rcd_quotients<QUICK>(wsum, weight, mean);
+    R0[i] = green + interpolate(dir, mean[1], mean[0]);
+    B2[i] = green + interpolate(dir, mean[3], mean[2]);
+  });
+  __syncthreads();
+}
+
 // `load`: QUAD_PLAIN (mirrored plain loads), QUAD_TMA_F32 or QUAD_TMA_U16
 // for windows inside the image; `convert`: the f32 box needs Clip or the
 // balance applied in shared memory.
@@ -428,12 +646,6 @@ __global__ void __launch_bounds__(RTHREADS, 1) rcd_kernel(const MosaicSource src
   float* const R0 = S.rgb[0] + 2;
   float* const G1 = S.rgb[1] + 2;
   float* const B2 = S.rgb[2] + 2;
-  float* const vh = S.vh + 2;
-  float* const vhp = S.hp[0] + 2;
-  float* const hhp = S.hp[1] + 2;
-  float* const pcd = S.hp[0];  // half planes (index / 2)
-  float* const qcd = S.hp[1];
-  float* const pq = S.pq;
   ClipTally tally;
   // ---- populate (rcd.rs:226-271): the window's balanced samples; the two
   //      colours of each row get the CFA values.
@@ -469,149 +681,68 @@ __global__ void __launch_bounds__(RTHREADS, 1) rcd_kernel(const MosaicSource src
     }
   }
   const uint16_t* raw_win = reinterpret_cast<const uint16_t*>(S.hp[0]);
-  for (int k = tid; k < RW * RW; k += RTHREADS) {
-    const int row = k / RW, col = k - row * RW;
-    const int i = row * RP + col;
-    const int ch = color_at(tp, col, row);
-    const bool core = row >= RB && row < RB + RT && col >= RB && col < RB + RT;
-    float n;
-    if (mode == QUAD_TMA_F32) {
-      n = cfa[i];
-    } else if (mode == QUAD_TMA_U16) {
-      const int sx = src.crop_x + wx + col, sy = src.crop_y + wy + row;
-      n = normalize_raw(src, (float)raw_win[row * RU + col + 6], sx, sy);
-    } else {
-      n = source_normalized(src, mirror_index(wx + col, W), mirror_index(wy + row, H));
-    }
-    float v = n;
-    if (mode != QUAD_TMA_F32 || convert) v = staged_value(src, n, ch);
-    if (count_clip && core && wx + col < W && wy + row < H) tally_value(tally, src, n, ch);
-    const int c0 = color_at(tp, 0, row), c1 = color_at(tp, 1, row);
-    cfa[i] = v;
-    R0[i] = (c0 == 0 || c1 == 0) ? v : 0.0f;
-    G1[i] = v;  // every row holds green
-    B2[i] = (c0 == 2 || c1 == 2) ? v : 0.0f;
-  }
-  __syncthreads();
-  // ---- squared high passes (rcd_stages.rs:8-48, 393-404): vertical at rows
-  //      [3, RW-3) x cols [4, RW-4), horizontal at rows [4, RW-4) x cols [3, RW-3)
-  for (int k = tid; k < (RW - 6) * (RW - 6); k += RTHREADS) {
-    const int r = 3 + k / (RW - 6), c = 3 + k % (RW - 6);
-    const int i = r * RP + c;
-    if (c >= 4 && c < RW - 4)
-      vhp[i] = rsq((cfa[i - 3 * RP] - cfa[i - RP] - cfa[i + RP] + cfa[i + 3 * RP]) -
-                   3.0f * (cfa[i - 2 * RP] + cfa[i + 2 * RP]) + 6.0f * cfa[i]);
-    if (r >= 4 && r < RW - 4)
-      hhp[i] = rsq((cfa[i - 3] - cfa[i - 1] - cfa[i + 1] + cfa[i + 3]) - 3.0f * (cfa[i - 2] + cfa[i + 2]) + 6.0f * cfa[i]);
-  }
-  __syncthreads();
-  // ---- find_directions (rcd_stages.rs:8-48) at [4, RW-4)^2 and the low pass
-  //      (:55-82) at the red/blue sites of [2, RW-2)^2
-  for (int k = tid; k < (RW - 8) * (RW - 8); k += RTHREADS) {
-    const int r = 4 + k / (RW - 8), c = 4 + k % (RW - 8);
-    const int i = r * RP + c;
-    const float vs = rmaxf(vhp[i - RP] + vhp[i] + vhp[i + RP], REPS2);
-    const float hs = rmaxf(hhp[i - 1] + hhp[i] + hhp[i + 1], REPS2);
-    vh[i] = vs / (vs + hs);
-  }
-  for (int k = tid; k < (RW - 4) * ((RW - 4) / 2); k += RTHREADS) {
-    const int r = 2 + k / ((RW - 4) / 2);
-    const int c = 2 + (color_at(tp, 0, r) & 1) + 2 * (k % ((RW - 4) / 2));
-    const int i = r * RP + c;
-    pq[i / 2] = cfa[i] + 0.5f * (cfa[i - RP] + cfa[i + RP] + cfa[i - 1] + cfa[i + 1]) +
-                0.25f * (cfa[i - RP - 1] + cfa[i - RP + 1] + cfa[i + RP - 1] + cfa[i + RP + 1]);
-  }
-  __syncthreads();
-  // ---- interpolate_green (rcd_stages.rs:84-147) at the red/blue sites of
-  //      [4, RW-4)^2; calculate_diagonal_high_pass (:162-196) at the odd
-  //      columns of [3, RW-3)^2 (into the high-pass area, now free)
-  constexpr int SITES4 = (RW - 8) / 2;  // red/blue sites per row of [4, RW-4)
-  for (int k = tid; k < (RW - 8) * SITES4; k += RTHREADS) {
-    const int r = 4 + k / SITES4;
-    const int c = 4 + (color_at(tp, 0, r) & 1) + 2 * (k % SITES4);
-    const int i = r * RP + c;
-    const float ng = cardinal_gradient(cfa, i, -RP), sg = cardinal_gradient(cfa, i, RP);
-    const float wg = cardinal_gradient(cfa, i, -1), eg = cardinal_gradient(cfa, i, 1);
-    const int li = i / 2;
-    const float lp = pq[li];
-    const float ne = ratio_estimate(cfa[i - RP], lp, pq[li - RP]);
-    const float se = ratio_estimate(cfa[i + RP], lp, pq[li + RP]);
-    const float we = ratio_estimate(cfa[i - 1], lp, pq[li - 1]);
-    const float ee = ratio_estimate(cfa[i + 1], lp, pq[li + 1]);
-    const float ve = weighted_pair(sg, ne, ng, se);
-    const float he = weighted_pair(wg, ee, eg, we);
-    const float dir = refined_direction(vh[i], vh[i - RP - 1], vh[i - RP + 1], vh[i + RP - 1], vh[i + RP + 1]);
-    G1[i] = interpolate(dir, he, ve);
-  }
-  constexpr int ODD3 = (RW - 6) / 2;  // odd columns of [3, RW-3)
-  for (int k = tid; k < (RW - 6) * ODD3; k += RTHREADS) {
-    const int r = 3 + k / ODD3, c = 3 + 2 * (k % ODD3);
-    const int i = r * RP + c;
-    pcd[i / 2] = rsq((cfa[i - 3 * RP - 3] - cfa[i - RP - 1] - cfa[i + RP + 1] + cfa[i + 3 * RP + 3]) -
-                     3.0f * (cfa[i - 2 * RP - 2] + cfa[i + 2 * RP + 2]) + 6.0f * cfa[i]);
-    qcd[i / 2] = rsq((cfa[i - 3 * RP + 3] - cfa[i - RP + 1] - cfa[i + RP - 1] + cfa[i + 3 * RP - 3]) -
-                     3.0f * (cfa[i - 2 * RP + 2] + cfa[i + 2 * RP - 2]) + 6.0f * cfa[i]);
-  }
-  __syncthreads();
-  // ---- calculate_diagonal_directions (rcd_stages.rs:198-225), into pq
-  for (int k = tid; k < (RW - 8) * SITES4; k += RTHREADS) {
-    const int r = 4 + k / SITES4;
-    const int c = 4 + (color_at(tp, 0, r) & 1) + 2 * (k % SITES4);
-    const int i = r * RP + c;
-    const int hi = i / 2, pr = (i - RP - 1) / 2, nr = (i + RP - 1) / 2;
-    const float ps = rmaxf(pcd[pr] + pcd[hi] + pcd[nr + 1], REPS2);
-    const float qs = rmaxf(qcd[pr + 1] + qcd[hi] + qcd[nr], REPS2);
-    pq[hi] = ps / (ps + qs);
-  }
-  __syncthreads();
-  // ---- interpolate_opposite_color (rcd_stages.rs:227-285)
-  for (int k = tid; k < (RW - 8) * SITES4; k += RTHREADS) {
-    const int r = 4 + k / SITES4;
-    const int c = 4 + (color_at(tp, 0, r) & 1) + 2 * (k % SITES4);
-    const int i = r * RP + c;
-    const int ch = 2 - color_at(tp, c, r);
-    const int hi = i / 2, pr = (i - RP - 1) / 2, nr = (i + RP - 1) / 2;
-    const float dir = refined_direction(pq[hi], pq[pr], pq[pr + 1], pq[nr], pq[nr + 1]);
-    float* const v = ch == 0 ? R0 : B2;
-    const float* g = G1;
-    const float nwg = diagonal_gradient(v, g, i, -RP - 1), neg = diagonal_gradient(v, g, i, -RP + 1);
-    const float swg = diagonal_gradient(v, g, i, RP - 1), seg = diagonal_gradient(v, g, i, RP + 1);
-    const float nwe = v[i - RP - 1] - g[i - RP - 1], nee = v[i - RP + 1] - g[i - RP + 1];
-    const float swe = v[i + RP - 1] - g[i + RP - 1], see = v[i + RP + 1] - g[i + RP + 1];
-    const float dp = weighted_pair(nwg, see, seg, nwe);
-    const float dq = weighted_pair(neg, swe, swg, nee);
-    v[i] = g[i] + interpolate(dir, dq, dp);
-  }
-  __syncthreads();
-  // ---- interpolate_at_green (rcd_stages.rs:287-355) at the green sites of [4, RW-4)^2
-  for (int k = tid; k < (RW - 8) * SITES4; k += RTHREADS) {
-    const int r = 4 + k / SITES4;
-    const int c = 4 + (color_at(tp, 1, r) & 1) + 2 * (k % SITES4);
-    const int i = r * RP + c;
-    const float dir = refined_direction(vh[i], vh[i - RP - 1], vh[i - RP + 1], vh[i + RP - 1], vh[i + RP + 1]);
-    const float* g = G1;
-    const float green = g[i];
-    const float n1 = REPS + fabsf(green - g[i - 2 * RP]);
-    const float s1 = REPS + fabsf(green - g[i + 2 * RP]);
-    const float w1 = REPS + fabsf(green - g[i - 2]);
-    const float e1 = REPS + fabsf(green - g[i + 2]);
-    const float gn = g[i - RP], gs = g[i + RP], gw = g[i - 1], ge = g[i + 1];
+  bool large = false;  // a sample outside QUICK's range
+  if (mode == QUAD_TMA_U16 && src.parity_levels) {
+    // By 2x2 cells, as in quad_kernel (the window origin is even).
+    float span_y[4];
 #pragma unroll
-    for (int chn = 0; chn <= 2; chn += 2) {
-      float* v = chn == 0 ? R0 : B2;
-      const float nsa = fabsf(v[i - RP] - v[i + RP]);
-      const float ewa = fabsf(v[i - 1] - v[i + 1]);
-      const float ngr = n1 + nsa + fabsf(v[i - RP] - v[i - 3 * RP]);
-      const float sgr = s1 + nsa + fabsf(v[i + RP] - v[i + 3 * RP]);
-      const float wgr = w1 + ewa + fabsf(v[i - 1] - v[i - 3]);
-      const float egr = e1 + ewa + fabsf(v[i + 1] - v[i + 3]);
-      const float ne = v[i - RP] - gn, se = v[i + RP] - gs, we = v[i - 1] - gw, ee = v[i + 1] - ge;
-      const float vert = weighted_pair(ngr, se, sgr, ne);
-      const float horiz = weighted_pair(egr, we, wgr, ee);
-      v[i] = green + interpolate(dir, horiz, vert);
+    for (int j = 0; j < 4; ++j) span_y[j] = reciprocal_of(src.level_span[j]);
+    constexpr int CW = RW / 2;
+    for (int k = tid; k < CW * CW; k += RTHREADS) {
+      const int row = 2 * (k / CW), col = 2 * (k % CW);
+      const unsigned top = *reinterpret_cast<const unsigned*>(raw_win + row * RU + col + 6);
+      const unsigned low = *reinterpret_cast<const unsigned*>(raw_win + (row + 1) * RU + col + 6);
+      const unsigned raw[4] = {top & 0xffffu, top >> 16, low & 0xffffu, low >> 16};
+      const bool core = count_clip && row >= RB && row < RB + RT && col >= RB && col < RB + RT;
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int ch = color_at(tp, j & 1, j >> 1);
+        const float n = normalize_parity(src, raw[j], j, span_y[j]);
+        v[j] = staged_value(src, n, ch);
+        if (core && wx + col + (j & 1) < W && wy + row + (j >> 1) < H) tally_value(tally, src, n, ch);
+      }
+      large = large || !(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))) <= 0x1p20f);
+      const bool red_top = color_at(tp, 0, 0) == 0 || color_at(tp, 1, 0) == 0;  // else blue
+#pragma unroll
+      for (int dy = 0; dy < 2; ++dy) {
+        const int i = (row + dy) * RP + col;
+        const float2 pair = make_float2(v[2 * dy], v[2 * dy + 1]), none = make_float2(0.0f, 0.0f);
+        const bool red = red_top == (dy == 0);
+        *reinterpret_cast<float2*>(cfa + i) = pair;
+        *reinterpret_cast<float2*>(R0 + i) = red ? pair : none;
+        *reinterpret_cast<float2*>(G1 + i) = pair;
+        *reinterpret_cast<float2*>(B2 + i) = red ? none : pair;
+      }
+    }
+  } else {
+    for (int k = tid; k < RW * RW; k += RTHREADS) {
+      const int row = k / RW, col = k - row * RW;
+      const int i = row * RP + col;
+      const int ch = color_at(tp, col, row);
+      const bool core = row >= RB && row < RB + RT && col >= RB && col < RB + RT;
+      float n;
+      if (mode == QUAD_TMA_F32) {
+        n = cfa[i];
+      } else if (mode == QUAD_TMA_U16) {
+        const int sx = src.crop_x + wx + col, sy = src.crop_y + wy + row;
+        n = normalize_raw(src, (float)raw_win[row * RU + col + 6], sx, sy);
+      } else {
+        n = source_normalized(src, mirror_index(wx + col, W), mirror_index(wy + row, H));
+      }
+      float v = n;
+      if (mode != QUAD_TMA_F32 || convert) v = staged_value(src, n, ch);
+      if (count_clip && core && wx + col < W && wy + row < H) tally_value(tally, src, n, ch);
+      const int c0 = color_at(tp, 0, row), c1 = color_at(tp, 1, row);
+      large = large || !(fabsf(v) <= 0x1p20f);
+      cfa[i] = v;
+      R0[i] = (c0 == 0 || c1 == 0) ? v : 0.0f;
+      G1[i] = v;  // every row holds green
+      B2[i] = (c0 == 2 || c1 == 2) ? v : 0.0f;
     }
   }
-  __syncthreads();
+  if (__syncthreads_or(large)) rcd_stages<false>(S, tp);
+  else rcd_stages<true>(S, tp);
   // ---- write_tile (rcd.rs:275-308): the measured sample replaces its channel.
   const long long plane = (long long)W * H;
   bool bad = false;

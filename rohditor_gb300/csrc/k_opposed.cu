@@ -30,13 +30,11 @@
 // Every retry loop carries an iteration limit and reports through the error
 // word instead of spinning.
 #include <algorithm>
-#include <cmath>
 
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 #include <cuda_runtime.h>
 
-#include "quick_div.cuh"
 #include "rd_internal.cuh"
 
 namespace rd {
@@ -96,11 +94,6 @@ struct OpposedParams {
                              // [6] sites in the other tiles
   int tiles_x;               // estimate tiles per row
   unsigned* error;
-  // Raw samples whose levels depend on the position's parity only, with a plain
-  // span: the black level and the span (white - black) of the four positions of
-  // a cell; `parity_levels` says that they do.
-  int parity_levels;
-  float black[4], span[4];
 };
 
 __device__ __forceinline__ Cell load_cell(const OpposedParams& p, int x, int y) {
@@ -206,7 +199,7 @@ __device__ __forceinline__ void load_cell_samples(const OpposedParams& p, int cx
   const bool right = x + 1 < p.W, below = y + 1 < p.H;
   // Positions outside the image are neither suspected nor clean.
   v[1] = v[2] = v[3] = -INFINITY;
-  if (p.src.f32 || !p.parity_levels) {
+  if (p.src.f32 || !p.src.parity_levels) {
     v[0] = source_normalized(p.src, x, y);
     if (right) v[1] = source_normalized(p.src, x + 1, y);
     if (below) v[2] = source_normalized(p.src, x, y + 1);
@@ -228,9 +221,7 @@ __device__ __forceinline__ void load_cell_samples(const OpposedParams& p, int cx
   unsigned r[4] = {0u, 0u, 0u, 0u};
   pair(raw, r[0], r[1]);
   if (below) pair(raw + p.src.row_stride, r[2], r[3]);
-  auto normalized = [&](int k) {
-    return divide_by(__fsub_rn((float)r[k], p.black[k]), p.span[k], reciprocal_of(p.span[k]));
-  };
+  auto normalized = [&](int k) { return normalize_parity(p.src, r[k], k, reciprocal_of(p.src.level_span[k])); };
   v[0] = normalized(0);
   if (right) v[1] = normalized(1);
   if (below) v[2] = normalized(2);
@@ -1132,18 +1123,6 @@ Status run_opposed_labels(Context& ctx, const MosaicSource& src, float* mosaic, 
   p.stats = d_stats;
   p.counters = reinterpret_cast<unsigned*>(b + o_cnt);
   p.error = ctx.d_error;
-  // The levels of a cell's four positions, when the patterns repeat every one
-  // or two samples (cells start at even crop coordinates).
-  p.parity_levels = !src.f32 && src.black_w <= 2 && src.black_h <= 2;
-  for (int k = 0; k < 4 && p.parity_levels; ++k) {
-    const int sx = src.crop_x + (k & 1), sy = src.crop_y + (k >> 1);
-    const int bi = (sy % src.black_h) * src.black_w + sx % src.black_w;
-    const float white = src.white_count == 1 ? src.white[0]
-                                             : src.white[src.white_count == 3 ? color_at(src.sensor_cfa, sx, sy) : bi];
-    p.black[k] = src.black[bi];
-    p.span[k] = white - src.black[bi];
-    if (!((p.black[k] == 0.0f || std::fabs(p.black[k]) >= 0x1p-60f) && std::fabs(p.black[k]) <= 0x1p30f && p.span[k] >= 0x1p-30f && p.span[k] <= 0x1p30f)) p.parity_levels = 0;
-  }
   RD_CUDA_TRY(cudaMemsetAsync(b + o_bits, 0, bytes - o_bits, ctx.stream));
   const int sms = ctx.sm_count > 0 ? ctx.sm_count : 152;
   const dim3 cgrid((cw + 127) / 128, (chh + CELL_ROWS - 1) / CELL_ROWS);

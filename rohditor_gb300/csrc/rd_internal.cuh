@@ -17,6 +17,8 @@
 
 #include "../../include/rd_gpu.h"
 
+#include "quick_div.cuh"
+
 namespace rd {
 
 // ------------------------------------------------------------------ errors
@@ -222,6 +224,11 @@ struct MosaicSource {
   float fwd[3];           // balance multipliers (1,1,1 when not balanced)
   float black[RD_MAX_LEVEL_PATTERN];
   float white[RD_MAX_LEVEL_PATTERN];
+  // Levels that repeat every one or two samples, of plain magnitudes: the black
+  // level and the span (white - black) by the parity of the crop coordinates,
+  // index 2 (y & 1) + (x & 1). `parity_levels` says that they hold.
+  int parity_levels;
+  float level_black[4], level_span[4];
 };
 
 __host__ __device__ inline int color_at(int pattern, int x, int y) {
@@ -254,6 +261,16 @@ __device__ __forceinline__ float normalize_raw(const MosaicSource& s, float samp
   else if (s.white_count == 3) white = s.white[color_at(s.sensor_cfa, sx, sy)];
   else white = s.white[bi];
   return __fdiv_rn(__fsub_rn(sample, black), __fsub_rn(white, black));
+}
+
+// Fills the levels by parity in (host).
+void set_parity_levels(MosaicSource& s);
+
+// normalize_raw by parity levels: position k of a 2x2 cell whose first sample
+// lies at even crop coordinates, y the span's reciprocal_of. Numerators are 0 or
+// at least 2^-60, spans between 2^-30 and 2^30, so the quotient is divide_by's.
+__device__ __forceinline__ float normalize_parity(const MosaicSource& s, unsigned sample, int k, float y) {
+  return divide_by(__fsub_rn((float)sample, s.level_black[k]), s.level_span[k], y);
 }
 
 // Normalized sample at crop coordinates (x, y) before any highlight step:
