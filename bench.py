@@ -194,9 +194,9 @@ def family_bytes(name: str, N: int, n: int) -> float | None:
     """Algorithmic bytes of one launch of a kernel family (N input pixels, n preview pixels)."""
     table = {
         "amaze": 14.0 * N,          # u16 mosaic in, planar f32 RGB out
-        "rl_iteration": 12.0 * N,   # estimate in, guide in, estimate out
+        "rl_iteration": 12.0 * N,   # estimate in, guide in, estimate out (the last one, with the gain: 36)
         "rl_mask": 20.0 * N,        # guide + mask preparation: RGB in, guide + refined mask out
-        "rl_apply": 36.0 * N,
+        "rl_apply": 36.0 * N,       # the gain of images below 256 x 64
         "vignetting": 4.0 * N,      # multiplier plane out
         "optics_gather": 28.0 * N,  # RGB + multiplier in, RGB out
         "area_reduce": 12.0 * N + 12.0 * n,  # RGB in, reduced RGB out (one pass)

@@ -13,9 +13,9 @@
 //                -> estimate = clamp(estimate * b, guide/2, 2 guide)
 //                so an iteration reads the estimate and guide once and writes
 //                the estimate once (12 bytes per pixel of compulsory traffic);
-//   rl_step      the same iteration with constant row lags for images of at
-//                least 256 x 64 (fewer instructions per row, see below);
-//   rl_apply     the bounded common RGB gain;
+//   rl_strip     the same iteration in the registers of a warp for images of at
+//                least 256 x 64 (see below); the last one applies the gain;
+//   rl_apply     the bounded common RGB gain of the smaller images;
 //   vignette_scan / vignette_plane  the exact incremental radius scan and the
 //                vignetting multiplier plane the optics gather reads.
 // Every blur keeps the reference's tap order (horizontal pass, then vertical,
@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -481,19 +482,41 @@ __device__ __forceinline__ void strip_item(int idx, int strips, int segs, int& s
 //  * A sum starts from its first product instead of from zero: every value of
 //    the iteration is positive (estimate >= guide / 2 > 0, ratio >= 0, taps >
 //    0), and 0 + p = p for every such p, so the sums are unchanged.
+//  * The last iteration has a row's new estimate and its guide in registers, so
+//    it applies the gain to the pixels there and stores no estimate: 36 bytes a
+//    pixel in one pass instead of 12 and 36 in two. Its own copies of a row's
+//    pixels and mask start before the row's blurs and need 20 registers, which
+//    R <= 3 has room for in the same 16 warps an SM.
 //
 // Measured at 6048 x 4024, R = 3 (radius 0.7): 74 us an iteration, 105 us with
 // the stages in shared memory (four barriers for 8 rows, 108 instructions a
 // pixel against 72). The estimate and the guide read once and the estimate
 // written take 44 us; the separately rounded products and sums (4 passes of 13
 // or 10, the ratio) 43 us of the FP32 pipe with the margins counted. 11648 x
-// 8736: 264 us (360); 512 x 344: 9.7 us (20).
+// 8736: 264 us (360); 512 x 344: 9.7 us (20). The last iteration with the gain at
+// 6048 x 4024: 171 us (74 and 154 as two launches; 36 bytes a pixel take 131 us).
 struct StepImage {
   const float* est_in;
   const float* guide;
   float* est_out;
   int W, H, strips, segs, items;
+  // The last iteration's launch applies the gain (sharpening.rs:110-118) itself.
+  float* rgb;
+  const float* mask;
+  float amount;
 };
+
+// The bounded common gain 1 + amount * mask * (est / guide - 1) on all three
+// channels, skipped when it is 1 or would make a channel non-finite.
+__device__ __forceinline__ bool apply_gain(float amount, float mask, float ratio, float& r, float& g, float& b) {
+  const float gain = 1.0f + amount * mask * (ratio - 1.0f);
+  const float v0 = r * gain, v1 = g * gain, v2 = b * gain;
+  if (!(gain != 1.0f && isfinite(v0) && isfinite(v1) && isfinite(v2))) return false;
+  r = v0;
+  g = v1;
+  b = v2;
+  return true;
+}
 
 template <int R>
 struct StripGeom {
@@ -502,6 +525,7 @@ struct StripGeom {
   static constexpr int AHEAD = 3;                          // steps in flight
   static constexpr int STEPS = 2 * R + AHEAD + 1;          // steps in the ring: of rows o .. o + 2R + AHEAD
   static constexpr int RESIDENT = R <= 3 ? 16 : 14;        // warps an SM holds: by registers, by the ring at R = 4
+  static constexpr int RESIDENT_APPLY = R <= 3 ? 16 : 12;  // with the pixels of a row in registers too
   static_assert(R <= 4, "a window reaches into the next lane only");
 };
 template <int R>
@@ -593,8 +617,9 @@ __device__ __forceinline__ float2 strip_feed(float2 (&acc)[2 * R], float2 h, con
 }
 
 // One work item (a strip and the rows [y0, y1) of segment seg) of one image's
-// iteration. INSIDE: the strip's 128 columns all lie in the image.
-template <int R, bool VEC, bool INSIDE>
+// iteration. INSIDE: the strip's 128 columns all lie in the image. APPLY: the
+// row's gain is applied to the pixels in place of storing the estimate.
+template <int R, bool VEC, bool INSIDE, bool APPLY>
 __device__ __forceinline__ void strip_rows(const StepImage& im, int xb, int seg, const float2 (&k2)[R + 1], float2 z,
                                            StripRing<R>& ring) {
   using G = StripGeom<R>;
@@ -682,6 +707,22 @@ __device__ __forceinline__ void strip_rows(const StepImage& im, int xb, int seg,
   };
   // The second blur: ratio row in, the finished row R above it out.
   auto blur2 = [&](const Quad h) { return Quad{strip_feed<R>(ua, h.a, k2, z), strip_feed<R>(ub, h.b, k2, z)}; };
+  // With APPLY: row o's pixels and mask, under way while its estimate is formed.
+  const long long plane = (long long)W * H;
+  float4 pixels[4];
+  auto pixel_row = [&](float* base) { return base + (long long)o * W + x; };
+  auto load_pixels = [&]() {
+    if (!APPLY || !store) return;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float* s = pixel_row(c < 3 ? im.rgb + c * plane : const_cast<float*>(im.mask));
+      if (VEC) {
+        pixels[c] = *reinterpret_cast<const float4*>(s);
+      } else {
+        pixels[c] = make_float4(s[0], x + 1 < W ? s[1] : 0.0f, x + 2 < W ? s[2] : 0.0f, x + 3 < W ? s[3] : 0.0f);
+      }
+    }
+  };
   // The bounded update of row o. The develop rejects non-finite capture input,
   // so nothing is NaN here, and min / max give the reference's
   // compare-and-replace.
@@ -693,7 +734,29 @@ __device__ __forceinline__ void strip_rows(const StepImage& im, int xb, int seg,
     const float n1 = fminf(fmaxf(eo.y * b.a.y, go.y * 0.5f), go.y * 2.0f);
     const float n2 = fminf(fmaxf(eo.z * b.b.x, go.z * 0.5f), go.z * 2.0f);
     const float n3 = fminf(fmaxf(eo.w * b.b.y, go.w * 0.5f), go.w * 2.0f);
-    if (store) {
+    if (APPLY && store) {
+      const float n[4] = {n0, n1, n2, n3}, gd[4] = {go.x, go.y, go.z, go.w};
+      float* px = &pixels[0].x;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float q = quick_div(n[j], gd[j]);
+        if (!(gd[j] <= 0x1p60f)) q = n[j] / gd[j];
+        apply_gain(im.amount, px[12 + j], q, px[j], px[4 + j], px[8 + j]);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        float* d = pixel_row(im.rgb + c * plane);
+        if (VEC) {
+          *reinterpret_cast<float4*>(d) = pixels[c];
+        } else {
+          d[0] = pixels[c].x;
+          if (x + 1 < W) d[1] = pixels[c].y;
+          if (x + 2 < W) d[2] = pixels[c].z;
+          if (x + 3 < W) d[3] = pixels[c].w;
+        }
+      }
+    }
+    if (!APPLY && store) {
       float* d = reinterpret_cast<float*>(const_cast<char*>(out.row(o)));
       if (VEC) {
         *reinterpret_cast<float4*>(d) = make_float4(n0, n1, n2, n3);
@@ -722,23 +785,27 @@ __device__ __forceinline__ void strip_rows(const StepImage& im, int xb, int seg,
 #pragma unroll 1
   while (r < r_end) {
     const int row = r;
+    load_pixels();
     const Quad h = ratio(blur1());
     if (row >= keep_from) keep(H - 1 - row, h);
     update(blur2(h));
   }
   if (bottom) {
 #pragma unroll 1
-    for (int i = 0; i < R; ++i) update(blur2(kept(i)));
+    for (int i = 0; i < R; ++i) {
+      load_pixels();
+      update(blur2(kept(i)));
+    }
   }
 }
-template <int R, bool VEC>
+template <int R, bool VEC, bool APPLY>
 __device__ __forceinline__ void strip_step(const StepImage& im, int item, const float2 (&k2)[R + 1], float2 z,
                                            StripRing<R>& ring) {
   int strip, seg;
   strip_item(item, im.strips, im.segs, strip, seg);
   const int xb = strip * StripGeom<R>::OUT - 4 * StripGeom<R>::MARGIN;
-  if (xb >= 0 && xb + 128 <= im.W) strip_rows<R, VEC, true>(im, xb, seg, k2, z, ring);
-  else strip_rows<R, VEC, false>(im, xb, seg, k2, z, ring);
+  if (xb >= 0 && xb + 128 <= im.W) strip_rows<R, VEC, true, APPLY>(im, xb, seg, k2, z, ring);
+  else strip_rows<R, VEC, false, APPLY>(im, xb, seg, k2, z, ring);
 }
 
 template <int R>
@@ -752,23 +819,25 @@ struct StripTaps {
 };
 
 // One warp a block, so that rows, loop counts and row addresses are uniform.
-template <int R, bool VEC>
-__global__ void __launch_bounds__(32, StripGeom<R>::RESIDENT) rl_strip_kernel(const StepImage im, const Taps taps) {
+template <int R, bool VEC, bool APPLY>
+__global__ void __launch_bounds__(32, APPLY ? StripGeom<R>::RESIDENT_APPLY : StripGeom<R>::RESIDENT)
+    rl_strip_kernel(const StepImage im, const Taps taps) {
   __shared__ StripRing<R> ring;
   const StripTaps<R> t(taps);
-  strip_step<R, VEC>(im, blockIdx.x, t.k2, t.z, ring);
+  strip_step<R, VEC, APPLY>(im, blockIdx.x, t.k2, t.z, ring);
 }
 
 // One iteration of several images in one launch (the batched develop's flat
-// pass): work items image by image in the table's order; first_item[i] is image
-// i's first item (first_item[n] = items). The images share the taps.
-template <int R, bool VEC>
-__global__ void __launch_bounds__(32, StripGeom<R>::RESIDENT)
+// pass): work items image by image in the table's order; image i's are
+// first_item[i] .. first_item[i + 1] - 1, counted from first_item[0]. The images
+// share the taps. APPLY: it is the last iteration of all of them.
+template <int R, bool VEC, bool APPLY>
+__global__ void __launch_bounds__(32, APPLY ? StripGeom<R>::RESIDENT_APPLY : StripGeom<R>::RESIDENT)
     rl_strip_images_kernel(const StepImage* __restrict__ images, const int* __restrict__ first_item, int nimages,
                            const Taps taps) {
   __shared__ StripRing<R> ring;
   const StripTaps<R> t(taps);
-  const int item = blockIdx.x;
+  const int item = first_item[0] + blockIdx.x;
   int lo = 0, hi = nimages;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -776,7 +845,7 @@ __global__ void __launch_bounds__(32, StripGeom<R>::RESIDENT)
     else hi = mid;
   }
   const StepImage im = images[lo];
-  strip_step<R, VEC>(im, item - first_item[lo], t.k2, t.z, ring);
+  strip_step<R, VEC, APPLY>(im, item - first_item[lo], t.k2, t.z, ring);
 }
 
 // Images of at least 256 x 64; smaller ones keep rl_stream_kernel, which copes
@@ -794,7 +863,7 @@ int strip_count(int W, int R) {
 template <int R>
 int strip_slots(int sms) {  // resident warps of the device
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_strip_kernel<R, true>, 32, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, rl_strip_kernel<R, true, false>, 32, 0);
   cudaGetLastError();
   return std::max(1, occ) * std::max(1, sms);
 }
@@ -802,16 +871,32 @@ int strip_slots(int sms) {  // resident warps of the device
 // Vector loads and stores: 16-byte rows in planes that start on 16 bytes.
 bool strip_vector(const float* planes, int W) { return W % 4 == 0 && (reinterpret_cast<uintptr_t>(planes) & 15) == 0; }
 
+// The gain that a develop's last iteration applies; rgb null before that.
+struct GainStep {
+  float* rgb = nullptr;
+  const float* mask = nullptr;
+  float amount = 0.0f;
+};
+
 template <int R>
 Status launch_rl_strip(Context& ctx, const float* est, const float* guide, float* out, int W, int H, const Taps& taps,
-                       int want) {
+                       int want, const GainStep& gain) {
+  // The segment count fills rounds of RESIDENT warps an SM.
+  if (gain.rgb) want = std::max(1, want * StripGeom<R>::RESIDENT_APPLY / StripGeom<R>::RESIDENT);
   const int segs = strip_segments(H, want), strips = strip_count(W, R);
-  const StepImage im{est, guide, out, W, H, strips, segs, strips * segs};
-  // The two estimates and the guide are planes of one allocation.
-  if (strip_vector(est, W) && strip_vector(guide, W) && strip_vector(out, W)) {
-    RD_LAUNCH(ctx, K_RL_ITER, rl_strip_kernel<R, true><<<im.items, 32, 0, ctx.stream>>>(im, taps));
+  const StepImage im{est, guide, out, W, H, strips, segs, strips * segs, gain.rgb, gain.mask, gain.amount};
+  // The two estimates, the guide and the mask are planes of one allocation.
+  const bool vec = strip_vector(est, W) && strip_vector(guide, W) && strip_vector(out, W);
+  if (gain.rgb) {
+    if (vec && strip_vector(gain.rgb, W) && strip_vector(gain.mask, W)) {
+      RD_LAUNCH(ctx, K_RL_ITER, (rl_strip_kernel<R, true, true><<<im.items, 32, 0, ctx.stream>>>(im, taps)));
+    } else {
+      RD_LAUNCH(ctx, K_RL_ITER, (rl_strip_kernel<R, false, true><<<im.items, 32, 0, ctx.stream>>>(im, taps)));
+    }
+  } else if (vec) {
+    RD_LAUNCH(ctx, K_RL_ITER, (rl_strip_kernel<R, true, false><<<im.items, 32, 0, ctx.stream>>>(im, taps)));
   } else {
-    RD_LAUNCH(ctx, K_RL_ITER, rl_strip_kernel<R, false><<<im.items, 32, 0, ctx.stream>>>(im, taps));
+    RD_LAUNCH(ctx, K_RL_ITER, (rl_strip_kernel<R, false, false><<<im.items, 32, 0, ctx.stream>>>(im, taps)));
   }
   return Status{};
 }
@@ -1405,13 +1490,13 @@ bool make_plane_map(CUtensorMap* map, const float* plane, int W, int H, int box_
 }
 
 Status rl_iteration(Context& ctx, int r, const Taps& taps, const float* est, const float* guide, float* out, int W,
-                    int H, const CUtensorMap* est_map, int segs) {
+                    int H, const CUtensorMap* est_map, int segs, const GainStep& gain) {
   if (rl_uses_strip_kernel(W, H, r)) {
     switch (r) {
-      case 1: return launch_rl_strip<1>(ctx, est, guide, out, W, H, taps, segs);
-      case 2: return launch_rl_strip<2>(ctx, est, guide, out, W, H, taps, segs);
-      case 3: return launch_rl_strip<3>(ctx, est, guide, out, W, H, taps, segs);
-      case 4: return launch_rl_strip<4>(ctx, est, guide, out, W, H, taps, segs);
+      case 1: return launch_rl_strip<1>(ctx, est, guide, out, W, H, taps, segs, gain);
+      case 2: return launch_rl_strip<2>(ctx, est, guide, out, W, H, taps, segs, gain);
+      case 3: return launch_rl_strip<3>(ctx, est, guide, out, W, H, taps, segs, gain);
+      case 4: return launch_rl_strip<4>(ctx, est, guide, out, W, H, taps, segs, gain);
       default: break;
     }
   }
@@ -1486,11 +1571,10 @@ __global__ void __launch_bounds__(256) rl_apply_kernel(const ApplyParams p) {
   const long long o = (long long)blockIdx.x * 256 + threadIdx.x;
   if (o >= p.plane) return;
   float v0 = p.rgb[o], v1 = p.rgb[p.plane + o], v2 = p.rgb[2 * p.plane + o];
-  const float gain = 1.0f + p.amount * p.mask[o] * (p.est[o] / p.guide[o] - 1.0f);
-  if (gain != 1.0f && isfinite(v0 * gain) && isfinite(v1 * gain) && isfinite(v2 * gain)) {
-    p.rgb[o] = v0 * gain;
-    p.rgb[p.plane + o] = v1 * gain;
-    p.rgb[2 * p.plane + o] = v2 * gain;
+  if (apply_gain(p.amount, p.mask[o], p.est[o] / p.guide[o], v0, v1, v2)) {
+    p.rgb[o] = v0;
+    p.rgb[p.plane + o] = v1;
+    p.rgb[2 * p.plane + o] = v2;
   }
 }
 
@@ -1681,6 +1765,7 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
   // iteration reads the guide plane itself.
   const float* est = guide;
   Status st;
+  bool gained = false;
   if (capture) {
     // The RGB planes as one (W, 3H) tensor for the prep kernel's tensor copies.
     CUtensorMap rgb_map;
@@ -1707,7 +1792,7 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
     std::vector<int> cands;
     if (segs == 0) {
       segs = rl_default_segments(W, H, r, ctx.sm_count > 0 ? ctx.sm_count : 152);
-      if (!ctx.capturing && ctx.tune_runs.empty() && detail.iterations >= 2) cands = rl_candidates(H, segs);
+      if (!ctx.capturing && ctx.tune_runs.empty() && detail.iterations >= 3) cands = rl_candidates(H, segs);
     }
     if (!cands.empty()) {
       ctx.tune_shape[0] = W;
@@ -1715,7 +1800,13 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
       ctx.tune_shape[2] = r;
     }
     for (int it = 0; it < detail.iterations && st.ok(); ++it) {
-      const bool timed = !cands.empty() && it > 0;
+      // The last iteration of a strip image applies the gain too; it is not
+      // timed, being another kernel.
+      const bool last = it + 1 == detail.iterations;
+      GainStep gain;
+      if (last && rl_uses_strip_kernel(W, H, r)) gain = GainStep{rgb, mask, detail.amount};
+      gained = gain.rgb != nullptr;
+      const bool timed = !cands.empty() && it > 0 && !last;
       const int s_it = timed ? cands[(it - 1) % cands.size()] : segs;
       cudaEvent_t a = nullptr, b = nullptr;
       if (timed) {
@@ -1729,7 +1820,7 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
         }
         cudaEventRecord(a, ctx.stream);
       }
-      st = rl_iteration(ctx, r, taps, est, guide, est_buf[it & 1], W, H, in_map, s_it);
+      st = rl_iteration(ctx, r, taps, est, guide, est_buf[it & 1], W, H, in_map, s_it, gain);
       if (timed) {
         cudaEventRecord(b, ctx.stream);
         ctx.tune_runs.push_back({s_it, {a, b}});
@@ -1739,7 +1830,7 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
     }
     if (st.ok() && cudaGetLastError() != cudaSuccess) st = Status{RD_SYNCHRONIZATION, "capture kernels failed to launch"};
   }
-  if (st.ok()) {
+  if (st.ok() && !gained) {
     ApplyParams ap{};
     ap.rgb = rgb;
     ap.plane = plane;
@@ -1761,20 +1852,26 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
 namespace {
 
 template <int R, bool VEC>
-Status launch_rl_strip_images(Context& ctx, const StepImage* d_images, const int* d_first, int nimages, int items,
-                              const Taps& taps) {
-  RD_LAUNCH(ctx, K_RL_ITER,
-            rl_strip_images_kernel<R, VEC><<<items, 32, 0, ctx.stream>>>(d_images, d_first, nimages, taps));
+Status launch_rl_strip_images(Context& ctx, bool apply, const StepImage* d_images, const int* d_first, int nimages,
+                              int items, const Taps& taps) {
+  if (apply) {
+    RD_LAUNCH(ctx, K_RL_ITER,
+              (rl_strip_images_kernel<R, VEC, true><<<items, 32, 0, ctx.stream>>>(d_images, d_first, nimages, taps)));
+  } else {
+    RD_LAUNCH(ctx, K_RL_ITER,
+              (rl_strip_images_kernel<R, VEC, false><<<items, 32, 0, ctx.stream>>>(d_images, d_first, nimages, taps)));
+  }
   return Status{};
 }
 
-Status rl_strip_images(Context& ctx, int r, bool vec, const StepImage* d_images, const int* d_first, int nimages,
-                       int items, const Taps& taps) {
+Status rl_strip_images(Context& ctx, int r, bool vec, bool apply, const StepImage* d_images, const int* d_first,
+                       int nimages, int items, const Taps& taps) {
+  if (nimages == 0) return Status{};
   switch (r) {
-#define RD_STRIP_IMAGES_CASE(RR)                                                                       \
-  case RR:                                                                                            \
-    return vec ? launch_rl_strip_images<RR, true>(ctx, d_images, d_first, nimages, items, taps)        \
-               : launch_rl_strip_images<RR, false>(ctx, d_images, d_first, nimages, items, taps);
+#define RD_STRIP_IMAGES_CASE(RR)                                                                             \
+  case RR:                                                                                                  \
+    return vec ? launch_rl_strip_images<RR, true>(ctx, apply, d_images, d_first, nimages, items, taps)       \
+               : launch_rl_strip_images<RR, false>(ctx, apply, d_images, d_first, nimages, items, taps);
     RD_STRIP_IMAGES_CASE(1)
     RD_STRIP_IMAGES_CASE(2)
     RD_STRIP_IMAGES_CASE(3)
@@ -1845,7 +1942,7 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
       device_free(ctx, cp.planes, cp.bytes);
       continue;
     }
-    cp.vec = strip_vector(cp.planes, W);
+    cp.vec = strip_vector(cp.planes, W) && strip_vector(job.rgb, W);
     int segs = 0;
     {
       std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
@@ -1858,7 +1955,8 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
     prepared.push_back(cp);
   }
   // 2. The iterations: images with the same taps and row alignment
-  //    share one launch per iteration; an image leaves after its last one.
+  //    share one launch per iteration; those whose last one it is share another
+  //    (sharpening.rs:110-118: the gain) and leave.
   Status st;
   std::vector<bool> done(prepared.size(), false);
   for (size_t g = 0; g < prepared.size() && st.ok(); ++g) {
@@ -1884,62 +1982,61 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
     unsigned char* tb =
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(t) + 63) & ~static_cast<uintptr_t>(63));
     std::vector<unsigned char> host(table_bytes, 0);
-    std::vector<int> counts((size_t)max_k, 0), totals((size_t)max_k, 0);
+    // [it][0]: the images that go on, [it][1]: those that end; their number and work items.
+    struct Share {
+      int images = 0, items = 0;
+    };
+    std::vector<std::array<Share, 2>> shares((size_t)max_k);
     for (int it = 0; it < max_k; ++it) {
       StepImage* images = reinterpret_cast<StepImage*>(host.data() + (size_t)it * (img_bytes + first_bytes));
       int* first = reinterpret_cast<int*>(host.data() + (size_t)it * (img_bytes + first_bytes) + img_bytes);
       int m = 0, items = 0;
-      for (size_t i = 0; i < group.size(); ++i) {
-        const CapturePlanes& cp = prepared[group[i]];
-        if (cp.iterations <= it) continue;
-        const CaptureJob& job = jobs[cp.job];
-        const long long plane = (long long)job.W * job.H;
-        float* est[2] = {cp.planes + 2 * plane, cp.planes + 3 * plane};
-        StepImage& im = images[m];
-        im.est_in = it == 0 ? cp.planes : est[(it - 1) & 1];
-        im.guide = cp.planes;
-        im.est_out = est[it & 1];
-        im.W = job.W;
-        im.H = job.H;
-        im.strips = strip_count(job.W, r);
-        im.segs = cp.segs;
-        im.items = im.strips * im.segs;
-        first[m] = items;
-        items += im.items;
-        ++m;
+      for (int ends = 0; ends < 2; ++ends) {
+        for (size_t i = 0; i < group.size(); ++i) {
+          const CapturePlanes& cp = prepared[group[i]];
+          if (cp.iterations <= it || (cp.iterations == it + 1) != (ends == 1)) continue;
+          const CaptureJob& job = jobs[cp.job];
+          const long long plane = (long long)job.W * job.H;
+          float* est[2] = {cp.planes + 2 * plane, cp.planes + 3 * plane};
+          StepImage& im = images[m];
+          im.est_in = it == 0 ? cp.planes : est[(it - 1) & 1];
+          im.guide = cp.planes;
+          im.est_out = est[it & 1];
+          im.W = job.W;
+          im.H = job.H;
+          im.strips = strip_count(job.W, r);
+          im.segs = cp.segs;
+          im.items = im.strips * im.segs;
+          im.rgb = job.rgb;
+          im.mask = cp.planes + plane;
+          im.amount = job.detail.amount;
+          first[m] = items;
+          items += im.items;
+          shares[(size_t)it][ends].images += 1;
+          shares[(size_t)it][ends].items += im.items;
+          ++m;
+        }
       }
       first[m] = items;
-      counts[(size_t)it] = m;
-      totals[(size_t)it] = items;
     }
     st = upload(ctx, tb, host.data(), table_bytes);
     for (int it = 0; it < max_k && st.ok(); ++it) {
       const unsigned char* base = tb + (size_t)it * (img_bytes + first_bytes);
-      st = rl_strip_images(ctx, r, vec, reinterpret_cast<const StepImage*>(base),
-                          reinterpret_cast<const int*>(base + img_bytes), counts[(size_t)it], totals[(size_t)it],
-                          prepared[g].taps);
+      const StepImage* images = reinterpret_cast<const StepImage*>(base);
+      const int* first = reinterpret_cast<const int*>(base + img_bytes);
+      for (int ends = 0; ends < 2 && st.ok(); ++ends) {
+        const Share& sh = shares[(size_t)it][ends];
+        st = rl_strip_images(ctx, r, vec, ends == 1, images, first, sh.images, sh.items, prepared[g].taps);
+        images += sh.images;
+        first += sh.images;
+      }
     }
     if (st.ok() && cudaGetLastError() != cudaSuccess) st = Status{RD_SYNCHRONIZATION, "capture kernels failed to launch"};
     device_free(ctx, t, table_bytes + 64);
   }
-  // 3. The gain, image by image (sharpening.rs:110-118), then the planes go.
+  // 3. The planes go.
   for (CapturePlanes& cp : prepared) {
-    CaptureJob& job = jobs[cp.job];
-    const long long plane = (long long)job.W * job.H;
-    if (st.ok()) {
-      ApplyParams ap{};
-      ap.rgb = job.rgb;
-      ap.plane = plane;
-      ap.W = job.W;
-      ap.H = job.H;
-      ap.amount = job.detail.amount;
-      ap.mask = cp.planes + plane;
-      ap.est = cp.planes + (2 + ((cp.iterations - 1) & 1)) * plane;
-      ap.guide = cp.planes;
-      RD_LAUNCH(ctx, K_RL_APPLY, rl_apply_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, ctx.stream>>>(ap));
-      if (cudaGetLastError() != cudaSuccess) st = Status{RD_SYNCHRONIZATION, "capture apply failed to launch"};
-    }
-    if (!st.ok()) job.st = st;
+    if (!st.ok()) jobs[cp.job].st = st;
     device_free(ctx, cp.planes, cp.bytes);
   }
   return st;

@@ -48,3 +48,16 @@ def test_ceiling_ranges(stages, oracle, ceilings):
     rng = np.random.default_rng(4)
     rgb = rng.uniform(-0.2, 1.5, size=(66, 3 * 260)).astype(np.float32)
     run(stages, oracle, rgb, 0.7, 0.3, ceilings, 2)
+
+
+@pytest.mark.parametrize("iterations", [1, 2])
+@pytest.mark.parametrize("width", [256, 333, 452])
+@pytest.mark.parametrize("radius", RADII)
+def test_gain_of_the_last_iteration(stages, oracle, radius, width, iterations):
+    # The last iteration applies the gain itself: levels whose gained channels
+    # overflow stay as they are, levels above 2^60 take the plain division.
+    rng = np.random.default_rng(width + iterations)
+    rgb = rng.uniform(-0.2, 1.5, size=(67, 3 * width)).astype(np.float32)
+    rgb[20:26, 90:300] *= np.float32(2.0**61)
+    rgb[40:44, 120:180] = rng.choice(np.float32([3.4e38, -3.4e38, 0.0]), size=(4, 60))
+    run(stages, oracle, rgb, radius, 0.2, (1.0, 0.9, 1.1), iterations)
