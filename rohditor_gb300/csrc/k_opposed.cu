@@ -192,7 +192,9 @@ __device__ __forceinline__ int pattern_position(int ch, unsigned support) {
 // cell. A thread takes CELL_ROWS cells of a column, all samples loaded before
 // the first is used. 11648 x 8736: 0.49 ms with a generic cell per thread, four
 // IEEE divisions and level look-ups each, 0.29 now; reading the samples and
-// writing mosaic and cells takes 0.16.
+// writing mosaic and cells takes 0.16. A block takes its places in the tile list
+// with one atomic: with hot pixels all over, an atomic per tile on that one
+// counter kept the kernel at 0.49.
 constexpr int CELL_ROWS = 4;
 __device__ __forceinline__ void load_cell_samples(const OpposedParams& p, int cx, int cy, float (&v)[4]) {
   const int x = 2 * cx, y = 2 * cy;
@@ -229,7 +231,8 @@ __device__ __forceinline__ void load_cell_samples(const OpposedParams& p, int cx
 }
 
 __global__ void __launch_bounds__(128) cells_kernel(const OpposedParams p) {
-  __shared__ unsigned block_counts[4];
+  __shared__ unsigned block_counts[4];  // suspected sites per channel, then the tiles to list
+  __shared__ unsigned new_tiles[128 / ETX], list_at;
   if (threadIdx.x < 4) block_counts[threadIdx.x] = 0;
   __syncthreads();
   const int cx = blockIdx.x * blockDim.x + threadIdx.x, cy0 = blockIdx.y * CELL_ROWS;
@@ -276,16 +279,21 @@ __global__ void __launch_bounds__(128) cells_kernel(const OpposedParams p) {
       p.suspected[i] = (unsigned char)suspected;
       if (suspected) {
         packed += (sr ? 1u : 0u) + (sg0 ? 1u << 8 : 0u) + (sg1 ? 1u << 8 : 0u) + (sb ? 1u << 16 : 0u);
-        // Count the cell's sites in its estimate tile; the first ones append the tile to the list.
-        const unsigned tile = (unsigned)((cy / ETY) * p.tiles_x + cx / ETX);
-        const unsigned sites = (sr ? 1u : 0u) + (sg0 ? 1u : 0u) + (sg1 ? 1u : 0u) + (sb ? 1u : 0u);
-        if (atomicAdd(&p.tile_sites[tile], sites) == 0u) p.tile_list[atomicAdd(&p.counters[2], 1u)] = tile;
       }
     }
   }
   // A thread counts at most 2 CELL_ROWS sites of a channel, a warp 32 times that: the fields are widened first.
   const unsigned FULL = 0xffffffffu;
   if (__any_sync(FULL, packed != 0u)) {
+    // The sites of a thread are counted in their estimate tile once for the lanes
+    // of its columns; the first ones append the tile to the list.
+    static_assert(ETY % CELL_ROWS == 0 && ETX <= 32 && (ETX & (ETX - 1)) == 0, "a thread's cells lie in one tile");
+    const unsigned tile_lanes = (FULL >> (32 - ETX)) << (threadIdx.x & 31 & ~(unsigned)(ETX - 1));
+    const unsigned sites = __reduce_add_sync(tile_lanes, (packed & 255u) + (packed >> 8 & 255u) + (packed >> 16));
+    if (sites && (threadIdx.x & (ETX - 1)) == 0) {
+      const unsigned tile = (unsigned)((cy0 / ETY) * p.tiles_x + cx / ETX);
+      if (atomicAdd(&p.tile_sites[tile], sites) == 0u) new_tiles[atomicAdd(&block_counts[3], 1u)] = tile;
+    }
     const unsigned red_blue = __reduce_add_sync(FULL, packed & 0x00ff00ffu), green = __reduce_add_sync(FULL, (packed >> 8) & 255u);
     if ((threadIdx.x & 31) == 0) {
       atomicAdd(&block_counts[0], red_blue & 0xffffu);
@@ -294,58 +302,111 @@ __global__ void __launch_bounds__(128) cells_kernel(const OpposedParams p) {
     }
   }
   __syncthreads();
-  if (threadIdx.x < 3 && block_counts[threadIdx.x]) {
-    atomicAdd(&p.counters[0], block_counts[threadIdx.x]);
+  if (threadIdx.x < 3 && block_counts[threadIdx.x])
     atomicAdd(&p.stats[6 + threadIdx.x], (unsigned long long)block_counts[threadIdx.x]);
+  if (threadIdx.x == 3) {
+    const unsigned all = block_counts[0] + block_counts[1] + block_counts[2];
+    if (all) atomicAdd(&p.counters[0], all);
   }
+  const unsigned tiles = block_counts[3];
+  if (tiles == 0) return;
+  if (threadIdx.x == 0) list_at = atomicAdd(&p.counters[2], tiles);
+  __syncthreads();
+  if (threadIdx.x < tiles) p.tile_list[list_at + threadIdx.x] = new_tiles[threadIdx.x];
 }
 
-// 3. dilation + union-find initialisation, DILATE_CELLS cells of a row per
-// thread (their 3x3 neighbourhoods share columns, and the loads of a thread
-// are independent); the inside cells are appended to the cell list, one
-// atomic per warp.
-constexpr int DILATE_CELLS = 4;
-__global__ void __launch_bounds__(128) dilate_kernel(const OpposedParams p) {
+// 3. dilation + union-find initialisation, a block of DILATE_CELLS x
+// DILATE_ROWS cells per thread (their 3x3 neighbourhoods share columns and rows,
+// and the loads of a thread are independent); the inside cells are appended to
+// the cell list, row by row within a warp and with one atomic per block: where
+// most warps have some, an atomic each on the one counter is what the kernel
+// waits for. 11648 x 8736: 226 us with a row per thread and an atomic per warp,
+// 50 now.
+constexpr int DILATE_CELLS = 4, DILATE_ROWS = 4, DILATE_THREADS = 128;
+__global__ void __launch_bounds__(DILATE_THREADS) dilate_kernel(const OpposedParams p) {
   if (p.counters[0] == 0) return;
-  const int cx0 = (blockIdx.x * blockDim.x + threadIdx.x) * DILATE_CELLS, cy = blockIdx.y;
-  unsigned inside = 0;  // bit j: cell cx0 + j is inside
+  __shared__ unsigned warp_total[DILATE_THREADS / 32], list_at;
+  const int cx0 = (blockIdx.x * blockDim.x + threadIdx.x) * DILATE_CELLS, cy0 = blockIdx.y * DILATE_ROWS;
+  unsigned inside = 0;  // bit DILATE_CELLS * row + j: cell (cx0 + j, cy0 + row) is inside
   if (cx0 < p.cw) {
-    const int y0 = max(cy - 1, 0), y1 = min(cy + 1, p.ch - 1);
-    unsigned cols = 0;  // bit k: column cx0 - 1 + k holds a suspected cell in rows y0..y1
+    // Rows cy0 - 1 .. cy0 + DILATE_ROWS, per row a bit for each column cx0 - 1 + k with a suspected cell.
+    unsigned held[DILATE_ROWS + 2];
 #pragma unroll
-    for (int k = 0; k < DILATE_CELLS + 2; ++k) {
-      const int x = cx0 - 1 + k;
-      if (x < 0 || x >= p.cw) continue;
-      unsigned v = 0;
-      for (int y = y0; y <= y1; ++y) v |= p.suspected[(long long)y * p.cw + x];
-      if (v) cols |= 1u << k;
+    for (int r = 0; r < DILATE_ROWS + 2; ++r) {
+      const int y = cy0 - 1 + r;
+      held[r] = 0;
+      if (y < 0 || y >= p.ch) continue;
+      const unsigned char* row = p.suspected + (long long)y * p.cw;
+#pragma unroll
+      for (int k = 0; k < DILATE_CELLS + 2; ++k) {
+        const int x = cx0 - 1 + k;
+        if (x >= 0 && x < p.cw && row[x]) held[r] |= 1u << k;
+      }
     }
 #pragma unroll
-    for (int j = 0; j < DILATE_CELLS; ++j) {
-      const int x = cx0 + j;
-      if (x >= p.cw) break;
-      const bool in = ((cols >> j) & 7u) != 0;  // columns x - 1, x, x + 1
-      const long long i = (long long)cy * p.cw + x;
-      p.dilated[i] = in;
-      if (in) {
-        p.parent[i] = (unsigned)i;
-        inside |= 1u << j;
+    for (int r = 0; r < DILATE_ROWS; ++r) {
+      if (cy0 + r >= p.ch) break;
+      const unsigned cols = held[r] | held[r + 1] | held[r + 2];
+      const long long i = (long long)(cy0 + r) * p.cw + cx0;
+#pragma unroll
+      for (int j = 0; j < DILATE_CELLS; ++j) {
+        if (cx0 + j >= p.cw) break;
+        const bool in = ((cols >> j) & 7u) != 0;  // columns x - 1, x, x + 1
+        p.dilated[i + j] = in;
+        if (in) inside |= 1u << (DILATE_CELLS * r + j);
+      }
+    }
+    // The inside cells of an aligned 2x2 block touch each other: all link to the first.
+#pragma unroll
+    for (int r = 0; r < DILATE_ROWS; ++r) {
+      const long long i = (long long)(cy0 + r) * p.cw + cx0;
+#pragma unroll
+      for (int j = 0; j < DILATE_CELLS; ++j) {
+        if (!(inside & (1u << (DILATE_CELLS * r + j)))) continue;
+        const unsigned top = inside >> (DILATE_CELLS * (r & ~1) + (j & ~1)) & 3u;
+        const unsigned low = inside >> (DILATE_CELLS * (r | 1) + (j & ~1)) & 3u;
+        const int x = (j & ~1) + ((top ? top : low) & 1u ? 0 : 1);
+        p.parent[i + j] = (unsigned)(i + x - (top && (r & 1) ? p.cw : 0));
       }
     }
   }
-  const unsigned FULL = 0xffffffffu, lane = threadIdx.x & 31;
-  const unsigned n = __popc(inside);
+  // Counts of the four rows side by side, 8 bits each: a warp's row has at most 128 cells.
+  static_assert(DILATE_ROWS == 4 && 32 * DILATE_CELLS < 256, "a byte per row");
+  const unsigned FULL = 0xffffffffu, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned n = 0;
+#pragma unroll
+  for (int r = 0; r < DILATE_ROWS; ++r) n |= (unsigned)__popc(inside >> (DILATE_CELLS * r) & 15u) << (8 * r);
   unsigned incl = n;
   for (int off = 1; off < 32; off <<= 1) {
     const unsigned v = __shfl_up_sync(FULL, incl, off);
     if (lane >= (unsigned)off) incl += v;
   }
-  const unsigned total = __shfl_sync(FULL, incl, 31);
-  unsigned base = 0;
-  if (lane == 31 && total) base = atomicAdd(&p.counters[3], total);
-  base = __shfl_sync(FULL, base, 31) + incl - n;
-  for (int j = 0; j < DILATE_CELLS; ++j)
-    if (inside & (1u << j)) p.cell_list[base++] = (unsigned)((long long)cy * p.cw + cx0 + j);
+  const unsigned rows = __shfl_sync(FULL, incl, 31);
+  if (lane == 0) warp_total[warp] = (rows & 255u) + (rows >> 8 & 255u) + (rows >> 16 & 255u) + (rows >> 24);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned total = 0;
+#pragma unroll
+    for (int w = 0; w < DILATE_THREADS / 32; ++w) {
+      const unsigned t = warp_total[w];
+      warp_total[w] = total;
+      total += t;
+    }
+    if (total) list_at = atomicAdd(&p.counters[3], total);
+  }
+  __syncthreads();
+  if (inside == 0) return;
+  unsigned base = list_at + warp_total[warp];
+  const unsigned before = incl - n;
+#pragma unroll
+  for (int r = 0; r < DILATE_ROWS; ++r) {
+    unsigned at = base + (before >> (8 * r) & 255u);
+    const long long i = (long long)(cy0 + r) * p.cw + cx0;
+#pragma unroll
+    for (int j = 0; j < DILATE_CELLS; ++j)
+      if (inside & (1u << (DILATE_CELLS * r + j))) p.cell_list[at++] = (unsigned)(i + j);
+    base += rows >> (8 * r) & 255u;
+  }
 }
 
 // Root of i. Links only ever point to smaller indices, so shortening a path
@@ -385,17 +446,31 @@ __device__ void unite(unsigned* parent, unsigned a, unsigned b, unsigned* error)
   for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x, k##_n = p.counters[3]; k < k##_n; \
        k += gridDim.x * blockDim.x)
 
+// Links between the 2x2 blocks. A cell whose upper neighbour is inside needs no
+// other link of its own (that neighbour touches the other two above and the left
+// one); without it the left and the upper left one touch each other, the upper
+// right one neither (Wu, Otoo and Suzuki, Pattern Anal. Appl. 12, 2009). A
+// block's right column leaves out what its left column has linked already.
+// 6048 x 4024 with blown highlights: 47 us with a link to every neighbour from
+// single cells, 39 now; 11648 x 8736 with hot pixels: 307 and 156.
 __global__ void __launch_bounds__(256) union_kernel(const OpposedParams p) {
   FOR_LISTED_CELLS(k) {
     const unsigned i = p.cell_list[k];
     const unsigned cy = i / (unsigned)p.cw, cx = i - cy * (unsigned)p.cw;
-    if (cx > 0 && p.dilated[i - 1]) unite(p.parent, i, i - 1, p.error);
-    if (cy > 0) {
-      const unsigned up = i - p.cw;
-      if (cx > 0 && p.dilated[up - 1]) unite(p.parent, i, up - 1, p.error);
-      if (p.dilated[up]) unite(p.parent, i, up, p.error);
-      if (cx + 1 < (unsigned)p.cw && p.dilated[up + 1]) unite(p.parent, i, up + 1, p.error);
+    const unsigned up = i - p.cw;
+    const bool above = cy > 0, before = cx > 0;
+    const bool top = (cy & 1) == 0, left_column = (cx & 1) == 0;
+    if (above && p.dilated[up]) {
+      if (top && !(!left_column && p.dilated[i - 1] && p.dilated[up - 1])) unite(p.parent, i, up, p.error);
+      continue;
     }
+    if (before && p.dilated[i - 1]) {
+      if (left_column) unite(p.parent, i, i - 1, p.error);
+    } else if (above && before && p.dilated[up - 1]) {
+      if (top || left_column) unite(p.parent, i, up - 1, p.error);
+    }
+    if (above && cx + 1 < (unsigned)p.cw && p.dilated[up + 1] && (top || !left_column))
+      unite(p.parent, i, up + 1, p.error);
   }
 }
 
@@ -498,74 +573,133 @@ __global__ void clear_tables_kernel(const OpposedParams p) {
   }
 }
 
-// OR `bits` into word[key] once per distinct key of the warp (neighbouring
-// cells nearly always share their region).
-__device__ __forceinline__ void warp_or(unsigned* word, unsigned key, unsigned bits) {
-  namespace cg = cooperative_groups;
-  const cg::coalesced_group active = cg::coalesced_threads();
-  const cg::coalesced_group peers = cg::labeled_partition(active, key);
-  const unsigned v = cg::reduce(peers, bits, cg::bit_or<unsigned>());
-  if (peers.thread_rank() == 0 && v) atomicOr(&word[key], v);
-}
-
 // Final compact label of each dilated cell (1 + the roots before its root in
 // raster order), the per-region clipped channels, and 5. the wanted
 // (channel, support) slots per region (region_correction.rs:134-178), in one
 // pass: both need only the cell's own label. The sites of sparse estimate tiles
-// are listed on the way.
+// are listed on the way. Atomics are what it costs: neighbouring cells nearly
+// always share their region, so a warp's lanes find their equals once for both
+// tables, the union over the regions is kept in a register, and a block takes its
+// places in the site list at once. 11648 x 8736: 468 us with an atomic
+// each, 113 now.
 __global__ void __launch_bounds__(256) relabel_kernel(const OpposedParams p) {
-  FOR_LISTED_CELLS(k) {
-    const unsigned i = p.cell_list[k];
-    const unsigned r = p.labels[i], w = r >> 5;
-    unsigned label =
-        p.block_sums[w / RANK_BLOCK] + p.word_prefix[w] + __popc(p.root_bits[w] & ((1u << (r & 31)) - 1u)) + 1u;
-    if (label >= p.max_labels) {  // cannot happen for 8-connected regions of a 3x3 dilation
-      atomicOr(p.error, OPPOSED_ERROR);
-      label = 0;
-    }
-    p.labels[i] = label;
-    if (label == 0) continue;
-    const unsigned cy = i / (unsigned)p.cw, cx = i - cy * (unsigned)p.cw;
-    const Cell c = load_cell(p, (int)cx, (int)cy);
-    const unsigned clipped = c.flags >> 3;
-    if (clipped == 0) continue;
-    if (p.tile_sites[(cy / ETY) * (unsigned)p.tiles_x + cx / ETX] <= SPARSE_SITES) {
-      for (int q = 0; q < 4; ++q) {
-        const int x = 2 * (int)cx + (q & 1), y = 2 * (int)cy + (q >> 1);
-        if (x >= p.W || y >= p.H) continue;
-        const long long at = (long long)y * p.W + x;
-        if (p.mosaic[at] >= p.levels[color_at(p.cfa, x, y)]) p.site_list[atomicAdd(&p.counters[6], 1u)] = at;
+  const unsigned FULL = 0xffffffffu, lane = threadIdx.x & 31;
+  __shared__ unsigned warp_sites[8], site_at;
+  const unsigned cells = p.counters[3], stride = gridDim.x * blockDim.x, warp = threadIdx.x >> 5;
+  unsigned wanted_any = 0;
+  for (unsigned first = blockIdx.x * blockDim.x; first < cells; first += stride) {  // uniform in the block
+    const unsigned k = first + threadIdx.x;
+    unsigned label = 0, clipped = 0, bits = 0, sites = 0;  // sites: a bit per position of the cell
+    int x0 = 0, y0 = 0;
+    if (k < cells) {
+      const unsigned i = p.cell_list[k];
+      const unsigned r = p.labels[i], w = r >> 5;
+      label = p.block_sums[w / RANK_BLOCK] + p.word_prefix[w] + __popc(p.root_bits[w] & ((1u << (r & 31)) - 1u)) + 1u;
+      if (label >= p.max_labels) {  // cannot happen for 8-connected regions of a 3x3 dilation
+        atomicOr(p.error, OPPOSED_ERROR);
+        label = 0;
+      }
+      p.labels[i] = label;
+      const unsigned cy = i / (unsigned)p.cw, cx = i - cy * (unsigned)p.cw;
+      const Cell c = load_cell(p, (int)cx, (int)cy);
+      if (label != 0) clipped = c.flags >> 3;
+      if (clipped != 0) {
+        x0 = 2 * (int)cx;
+        y0 = 2 * (int)cy;
+        if (p.tile_sites[(cy / ETY) * (unsigned)p.tiles_x + cx / ETX] <= SPARSE_SITES) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int x = x0 + (q & 1), y = y0 + (q >> 1);
+            if (x < p.W && y < p.H && p.mosaic[(long long)y * p.W + x] >= p.levels[color_at(p.cfa, x, y)])
+              sites |= 1u << q;
+          }
+        }
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {
+          if (!(clipped & (1u << ch))) continue;
+          bool has_clean = false;
+          for (int o = 0; o < 3; ++o)
+            if (o != ch && usable(c, o) && clean(c, o)) has_clean = true;
+          if (!has_clean) continue;
+          const int pos = pattern_position(ch, support_mask(c, ch, p.levels));
+          if (pos >= 0) bits |= 1u << (ch * PATTERNS + pos);
+        }
       }
     }
-    warp_or(p.region_clipped, label, clipped);
-    unsigned bits = 0;
-    for (int ch = 0; ch < 3; ++ch) {
-      if (!(clipped & (1u << ch))) continue;
-      bool has_clean = false;
-      for (int o = 0; o < 3; ++o)
-        if (o != ch && usable(c, o) && clean(c, o)) has_clean = true;
-      if (!has_clean) continue;
-      const int pos = pattern_position(ch, support_mask(c, ch, p.levels));
-      if (pos >= 0) bits |= 1u << (ch * PATTERNS + pos);
+    wanted_any |= bits;
+    if (__any_sync(FULL, clipped != 0u)) {
+      const unsigned peers = __match_any_sync(FULL, label);
+      const unsigned all = __reduce_or_sync(peers, bits | clipped << SLOTS);
+      if (label != 0 && lane == (unsigned)(__ffs(peers) - 1) && all) {
+        atomicOr(&p.region_clipped[label], all >> SLOTS);
+        if (all & ((1u << SLOTS) - 1u)) atomicOr(&p.wanted[label], all & ((1u << SLOTS) - 1u));
+      }
     }
-    if (bits) {
-      warp_or(p.wanted, label, bits);
-      warp_or(p.wanted, 0u, bits);
+    if (__syncthreads_or(sites != 0u)) {
+      const unsigned n = __popc(sites);
+      unsigned incl = n;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned v = __shfl_up_sync(FULL, incl, off);
+        if (lane >= (unsigned)off) incl += v;
+      }
+      if (lane == 31) warp_sites[warp] = incl;
+      __syncthreads();
+      unsigned before = 0, total = 0;
+#pragma unroll
+      for (unsigned w = 0; w < 8; ++w) {
+        if (w < warp) before += warp_sites[w];
+        total += warp_sites[w];
+      }
+      if (threadIdx.x == 0) site_at = atomicAdd(&p.counters[6], total);
+      __syncthreads();
+      unsigned at = site_at + before + incl - n;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (sites & (1u << q)) p.site_list[at++] = (long long)(y0 + (q >> 1)) * p.W + x0 + (q & 1);
     }
   }
+  wanted_any = __reduce_or_sync(FULL, wanted_any);
+  if (lane == 0 && wanted_any) atomicOr(&p.wanted[0], wanted_any);
+}
+
+template <int N, int D>
+__device__ __forceinline__ void fold_sums(double* v, unsigned lane, int& at, int& size) {
+  constexpr int HALF = (N + 1) / 2;
+  const bool upper = (lane & D) != 0;
+#pragma unroll
+  for (int i = 0; i < HALF; ++i) {
+    const double hi = i + HALF < N ? v[i + HALF] : 0.0;
+    v[i] = (upper ? hi : v[i]) + __shfl_xor_sync(0xffffffffu, upper ? v[i] : hi, D);
+  }
+  at += upper ? HALF : 0;
+  size = upper ? size - HALF : min(size, HALF);
+  if constexpr (D > 1) fold_sums<HALF, D / 2>(v, lane, at, size);
 }
 
 // 6. region border statistics over the dilated cells; pass 0 = moments, pass
-// 1 = trimmed sums.
-__global__ void __launch_bounds__(256) border_kernel(const OpposedParams p, int pass) {
+// 1 = trimmed sums. The sums over all regions stay in a thread's registers and
+// reach shared memory once per warp and slot: adding doubles of 32 lanes to one
+// shared address is a loop of compare-and-swap, and the few warps that had
+// border cells kept the others at the last barrier. 6048 x 4024: 79 us
+// for the two passes so, 58 now (11648 x 8736 with hot pixels: 710 and 360).
+__global__ void __launch_bounds__(256, 3) border_kernel(const OpposedParams p, int pass) {
   if (p.counters[0] == 0) return;
-  __shared__ double pool[SLOTS][3];
+  __shared__ double pool[2 * SLOTS];
   __shared__ unsigned pool_n[SLOTS];
   if (threadIdx.x < SLOTS) {
-    pool[threadIdx.x][0] = pool[threadIdx.x][1] = pool[threadIdx.x][2] = 0.0;
+    pool[2 * threadIdx.x] = pool[2 * threadIdx.x + 1] = 0.0;
     pool_n[threadIdx.x] = 0;
   }
   __syncthreads();
+  const unsigned want_any = p.wanted[0], lane = threadIdx.x & 31;
+  unsigned mine_n[SLOTS];
+  double mine[SLOTS][2];
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) {
+    mine_n[s] = 0;
+    mine[s][0] = mine[s][1] = 0.0;
+  }
   FOR_LISTED_CELLS(k) {
     const unsigned i = p.cell_list[k];
     const unsigned label = p.labels[i];
@@ -574,12 +708,14 @@ __global__ void __launch_bounds__(256) border_kernel(const OpposedParams p, int 
     const Cell c = load_cell(p, (int)cx, (int)cy);
     if ((c.flags >> 3) == 0) {
       const unsigned rclip = p.region_clipped[label];
-      const unsigned want_r = p.wanted[label], want_any = p.wanted[0];
+      const unsigned want_r = p.wanted[label];
+#pragma unroll
       for (int ch = 0; ch < 3; ++ch) {
         if (!(rclip & (1u << ch))) continue;
         if (c.m[ch] < BORDER_MIN_FRACTION * p.levels[ch]) continue;
         unsigned pats[3];
         support_patterns(ch, pats);
+#pragma unroll
         for (int k = 0; k < 3; ++k) {
           const int off = ch * PATTERNS + k;
           const bool for_region = want_r & (1u << off);
@@ -587,55 +723,64 @@ __global__ void __launch_bounds__(256) border_kernel(const OpposedParams p, int 
           if (!for_region && !for_pool) continue;
           float value;
           if (!correction(c, ch, pats[k], p.levels, value)) continue;
-          float ratio = 0.0f;
-          const bool has_ratio = log_ratio(c, pats[k], ratio);
           const double wide = (double)value;
-          auto add = [&](long long slot, bool shared_pool) {
-            double* a = p.acc + slot * 4;
-            if (pass == 0) {
-              if (shared_pool) {
-                atomicAdd(&pool_n[off], 1u);
-                atomicAdd(&pool[off][0], wide);
-                atomicAdd(&pool[off][1], wide * wide);
-              } else {
-                atomicAdd(&a[0], 1.0);
-                atomicAdd(&a[2], wide);
-                atomicAdd(&a[3], wide * wide);
-              }
-            } else {
-              const float* t = p.trim + slot * 2;
-              if (fabsf(value - t[0]) <= t[1]) {
-                const double r = (double)(has_ratio ? ratio : 0.0f);
-                if (shared_pool) {
-                  atomicAdd(&pool_n[off], 1u);
-                  atomicAdd(&pool[off][0], wide);
-                  atomicAdd(&pool[off][2], r);
-                } else {
-                  atomicAdd(&a[1], 1.0);
-                  atomicAdd(&a[2], wide);
-                  atomicAdd(&a[3], r);
-                }
-              }
+          if (pass == 0) {
+            if (for_region) {
+              double* a = p.acc + ((long long)label * SLOTS + off) * 4;
+              atomicAdd(&a[0], 1.0);
+              atomicAdd(&a[2], wide);
+              atomicAdd(&a[3], wide * wide);
             }
-          };
-          if (for_region) add((long long)label * SLOTS + off, false);
-          if (for_pool) add(off, true);
+            if (for_pool) {
+              mine_n[off] += 1;
+              mine[off][0] += wide;
+              mine[off][1] += wide * wide;
+            }
+          } else {
+            float ratio = 0.0f;
+            const double r = log_ratio(c, pats[k], ratio) ? (double)ratio : 0.0;
+            auto kept = [&](long long slot) {
+              const float* t = p.trim + slot * 2;
+              return fabsf(value - t[0]) <= t[1];
+            };
+            const long long slot = (long long)label * SLOTS + off;
+            if (for_region && kept(slot)) {
+              double* a = p.acc + slot * 4;
+              atomicAdd(&a[1], 1.0);
+              atomicAdd(&a[2], wide);
+              atomicAdd(&a[3], r);
+            }
+            if (for_pool && kept(off)) {
+              mine_n[off] += 1;
+              mine[off][0] += wide;
+              mine[off][1] += r;
+            }
+          }
         }
       }
     }
   }
+  const unsigned FULL = 0xffffffffu;
+  unsigned any = 0;
+#pragma unroll
+  for (int s = 0; s < SLOTS; ++s) {
+    const unsigned n = __reduce_add_sync(FULL, mine_n[s]);
+    if (lane == 0 && n) atomicAdd(&pool_n[s], n);
+    any |= n;
+  }
+  if (any) {
+    // Each step hands half of the sums to the lane across and keeps the other
+    // half: 20 additions, and every lane ends with one sum, number `at`.
+    int at = 0, size = 2 * SLOTS;
+    fold_sums<2 * SLOTS, 16>(&mine[0][0], lane, at, size);
+    if (size > 0 && mine[0][0] != 0.0) atomicAdd(&pool[at], mine[0][0]);
+  }
   __syncthreads();
   if (threadIdx.x < SLOTS && pool_n[threadIdx.x]) {
     double* a = p.acc + threadIdx.x * 4;
-    if (pass == 0) {
-      atomicAdd(&a[0], (double)pool_n[threadIdx.x]);
-      atomicAdd(&a[2], pool[threadIdx.x][0]);
-      atomicAdd(&a[3], pool[threadIdx.x][1]);
-    } else {
-      atomicAdd(&a[1], (double)pool_n[threadIdx.x]);
-      atomicAdd(&a[2], pool[threadIdx.x][0]);
-      atomicAdd(&a[3], pool[threadIdx.x][2]);
-    }
+    atomicAdd(&a[pass == 0 ? 0 : 1], (double)pool_n[threadIdx.x]);
+    atomicAdd(&a[2], pool[2 * threadIdx.x]);
+    atomicAdd(&a[3], pool[2 * threadIdx.x + 1]);
   }
 }
 
@@ -1126,19 +1271,20 @@ Status run_opposed_labels(Context& ctx, const MosaicSource& src, float* mosaic, 
   RD_CUDA_TRY(cudaMemsetAsync(b + o_bits, 0, bytes - o_bits, ctx.stream));
   const int sms = ctx.sm_count > 0 ? ctx.sm_count : 152;
   const dim3 cgrid((cw + 127) / 128, (chh + CELL_ROWS - 1) / CELL_ROWS);
-  const dim3 dgrid((cw + 128 * DILATE_CELLS - 1) / (128 * DILATE_CELLS), chh);
+  const dim3 dgrid((cw + DILATE_THREADS * DILATE_CELLS - 1) / (DILATE_THREADS * DILATE_CELLS), (chh + DILATE_ROWS - 1) / DILATE_ROWS);
   const int lgrid = sms * 8;  // list kernels: 256-thread blocks, grid-stride
+  const int bgrid = sms * 3;  // as many as are resident: a block ends with a reduction in f64
   RD_LAUNCH(ctx, K_OPPOSED, cells_kernel<<<cgrid, 128, 0, ctx.stream>>>(p));
-  RD_LAUNCH(ctx, K_OPPOSED, dilate_kernel<<<dgrid, 128, 0, ctx.stream>>>(p));
+  RD_LAUNCH(ctx, K_OPPOSED, dilate_kernel<<<dgrid, DILATE_THREADS, 0, ctx.stream>>>(p));
   RD_LAUNCH(ctx, K_OPPOSED, union_kernel<<<lgrid, 256, 0, ctx.stream>>>(p));
   RD_LAUNCH(ctx, K_OPPOSED, flatten_kernel<<<lgrid, 256, 0, ctx.stream>>>(p));
   RD_LAUNCH(ctx, K_OPPOSED, rank_words_kernel<<<rank_blocks, RANK_BLOCK, 0, ctx.stream>>>(p, words));
   RD_LAUNCH(ctx, K_OPPOSED, scan_blocks_kernel<<<1, 1024, 0, ctx.stream>>>(p, rank_blocks));
   RD_LAUNCH(ctx, K_OPPOSED, clear_tables_kernel<<<sms * 2, 256, 0, ctx.stream>>>(p));
   RD_LAUNCH(ctx, K_OPPOSED, relabel_kernel<<<lgrid, 256, 0, ctx.stream>>>(p));
-  RD_LAUNCH(ctx, K_OPPOSED, border_kernel<<<lgrid, 256, 0, ctx.stream>>>(p, 0));
+  RD_LAUNCH(ctx, K_OPPOSED, border_kernel<<<bgrid, 256, 0, ctx.stream>>>(p, 0));
   RD_LAUNCH(ctx, K_OPPOSED, finish_moments_kernel<<<256, 256, 0, ctx.stream>>>(p));
-  RD_LAUNCH(ctx, K_OPPOSED, border_kernel<<<lgrid, 256, 0, ctx.stream>>>(p, 1));
+  RD_LAUNCH(ctx, K_OPPOSED, border_kernel<<<bgrid, 256, 0, ctx.stream>>>(p, 1));
   int dense_occ = 0, sparse_occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&dense_occ, estimate_dense_kernel, ETHREADS, 0) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sparse_occ, estimate_sparse_kernel, ETHREADS, 0) != cudaSuccess)
