@@ -189,10 +189,21 @@ RD_HD void chunk_tokens(const uint32_t* w, uint64_t breaks, int c0, int count, i
   uint32_t literal = all, match = 0;
   if (chunk_has_match(breaks, c0, count, before, after)) chunk_matches(breaks, c0, count, before, after, literal, match);
   if (literal == 0xFFFFFFFFu) {  // a whole chunk of literals, the common case
+    // A word at a time: its bytes are taken from it here, not all 32 in advance,
+    // which would not fit the registers.
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
-    for (int j = 0; j < CHUNK; ++j) visit(chunk_byte(w, j), 0);
+    for (int k = 0; k < CHUNK_WORDS; ++k) {
+      uint32_t word = w[k];
+#if defined(__CUDA_ARCH__)
+      asm volatile("" : "+r"(word)::"memory");
+#endif
+      visit(word & 0xFFu, 0);
+      visit((word >> 8) & 0xFFu, 0);
+      visit((word >> 16) & 0xFFu, 0);
+      visit(word >> 24, 0);
+    }
     return;
   }
   // The rare case word by word, the words moving up: a small loop, so that the
