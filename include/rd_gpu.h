@@ -171,8 +171,10 @@ uint64_t rd_ctx_kernel_launches(const rd_ctx* ctx);
  * shortens every wait, and `withhold` names a completion the next calls
  * never deliver: RD_WAIT_AMAZE_TILE (phase A of AMaZE tile 0 does not
  * publish its slab, so its phase B waits), RD_WAIT_RL_COPY (every block
- * of the capture-sharpening kernels skips its first tensor copy but waits
- * for it, then drains its other copies in flight), RD_WAIT_DEMOSAIC_COPY
+ * of the capture-sharpening kernels with tensor copies, which are the guide
+ * and mask pass and the iteration of images below 256 x 64, skips its first
+ * one but waits for it, then drains its other copies in flight),
+ * RD_WAIT_DEMOSAIC_COPY
  * (every block of the bilinear / MHC and RCD kernels skips the tensor copy
  * of its tile but waits for it; sources that TMA cannot address, and RCD
  * windows that cross the image edge, are staged by plain loads and have no
@@ -343,8 +345,9 @@ rd_status rd_encode_jpeg_device(rd_ctx* ctx, const uint8_t* d_rgb, uint32_t widt
  * suites (no reference counterpart). which = 0: the number of positive finite
  * f32 whose cube root is not correctly rounded (or not odd-symmetric), exact
  * integer comparison, expected 0. which = 1: the largest distance in ulps of
- * powf(x, 1/2.4) from the correctly rounded power over (0.0031308, 1], which
- * must not exceed the bound the 8- and 16-bit quantisation relies on (1).
+ * the transfer's estimate of x^(1/2.4) from the correctly rounded power over
+ * (0.0031308, 1], which must not exceed the bound that the 8- and 16-bit
+ * quantisation relies on (1).
  * which = 2: the number of f32 in (0.0031308, 1] whose transfer power (as the
  * quantisation computes it) differs from the correctly rounded one, expected 0.
  * which = 3: the number of (f32 in that domain, 8- or 16-bit, three dither

@@ -82,8 +82,6 @@ __device__ __forceinline__ int mirror_half(int index, int length) {
   return f < length ? f : 2 * length - 1 - f;
 }
 
-
-
 // ---- one RL iteration, streamed down column strips --------------------------
 // A CTA owns a strip of SW = 128 - 2R output columns and a segment of rows and
 // walks the segment top to bottom in steps of BH rows:

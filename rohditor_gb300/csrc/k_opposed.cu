@@ -31,8 +31,6 @@
 // word instead of spinning.
 #include <algorithm>
 
-#include <cooperative_groups.h>
-#include <cooperative_groups/reduce.h>
 #include <cuda_runtime.h>
 
 #include "rd_internal.cuh"

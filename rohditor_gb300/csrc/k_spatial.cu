@@ -4,9 +4,10 @@
 // Optics: the per-column and per-row halves of the pre-transform
 // (plan.rs:448-455 and correction.rs input_coordinate_x/y) are resolved on the
 // host in f64 and uploaded as f32 tables, so a pixel starts from two loads.
-// The inverse distortion runs the lensfun Newton iteration in f64 from the f32
-// coordinates (radius sqrt(f64(x*x + y*y)), <= 7 steps, |F| < 1e-5, input kept
-// on non-convergence; Poly3 returns NaN), TCA is applied in f32 and the
+// The inverse distortion has the values of the lensfun Newton iteration in f64
+// from the f32 coordinates (radius sqrt(f64(x*x + y*y)), <= 7 steps, |F| < 1e-5,
+// input kept on non-convergence; Poly3 returns NaN), computed in pairs of f32
+// wherever those decide the result (see below), TCA is applied in f32 and the
 // post-transform back to pixels is f64 narrowed once, as in
 // plan.rs:466-483. Each channel is a 4x4 Catmull-Rom gather with the
 // reference's tap order (resample.rs:21-33); a footprint outside [1, W-2]
