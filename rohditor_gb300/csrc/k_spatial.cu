@@ -176,8 +176,12 @@ __device__ __forceinline__ void undistort_poly5_fast(float x, float y, float a, 
   }
   const float d32 = 1.0f + 3.0f * a * s + 5.0f * b * (s * s);
   const float q32 = f0 / d32;
-  const float f1 = (3.0f * a * sq + 10.0f * b * sq * s) * q32 * q32;  // F(ru1) ~ F''/2 (F/F')^2
-  if (!(fabsf(f1) < 1.0e-6f) || !(d32 > 0.0f)) {
+  // F(ru1) for ru1 = rd - q, all of its terms: the second-order one vanishes at 3 k1 + 10 k2 u = 0. Their sum is good
+  // to 2^-21 of the largest, 5e-8 while that is below 0.1.
+  const float t2 = 3.0f * a * sq + 10.0f * b * sq * s, t3 = a + 10.0f * b * s, t4 = 5.0f * b * sq, q2 = q32 * q32;
+  const float f1 = (t2 - q32 * (t3 - q32 * (t4 - q32 * b))) * q2;
+  const float size = (fabsf(t2) + fabsf(q32) * (fabsf(t3) + fabsf(q32) * (fabsf(t4) + fabsf(q32 * b)))) * q2;
+  if (!(fabsf(f1) < 1.0e-6f) || !(size < 0.1f) || !(d32 > 0.0f)) {
     need_f64 = true;
     return;
   }
