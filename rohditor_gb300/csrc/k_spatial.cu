@@ -165,12 +165,15 @@ __device__ __forceinline__ void undistort_poly5_fast(float x, float y, float a, 
   oy = y;
   const float s = x * x + y * y;
   if (s == 0.0f) return;
-  const float g32 = a * s + b * (s * s);
+  const float as32 = a * s, bss32 = b * (s * s);
+  const float g32 = as32 + bss32;
   const float sq = sqrtf(s);
   const float f0 = sq * g32;
   const float thr = 1.0e-5f;
-  if (fabsf(f0) < thr * (1.0f - 1.0e-5f)) return;  // |F(rd)| < 1e-5: frozen at the input
-  if (fabsf(f0) <= thr * (1.0f + 1.0e-5f)) {
+  // f0 is good to a few 2^-24 of itself and of the two terms, which cancel where the distortion crosses zero.
+  const float off = thr * 1.0e-5f + sq * (fabsf(as32) + fabsf(bss32)) * 4.7683716e-7f;  // 2^-21
+  if (fabsf(f0) < thr - off) return;  // |F(rd)| < 1e-5: frozen at the input
+  if (fabsf(f0) <= thr + off) {
     need_f64 = true;
     return;
   }
