@@ -356,7 +356,11 @@ rd_status rd_encode_jpeg_device(rd_ctx* ctx, const uint8_t* d_rgb, uint32_t widt
  * over every f32 in [2^-12, 2), y hashed with 2^-18 <= |y| < 2, and y = 0)
  * whose hypot in the optics remap differs from f32::hypot as glibc computes
  * it (the double square root of the double sum of squares, narrowed once),
- * expected 0. */
+ * expected 0. which = 5: the number of sampled quotients (every significand of
+ * the divisor, hard and hashed numerators, both ends of the range) in which the
+ * kernels' division without special cases differs from the IEEE one, expected 0.
+ * which = 6: the same for its constant divisors, with every significand of the
+ * numerator, expected 0. */
 rd_status rd_check_math(rd_ctx* ctx, int32_t which, uint64_t* result);
 /* Launch shape of the capture-sharpening iteration chosen for one image shape
  * (no reference counterpart). The first develop of a (width, height, kernel

@@ -1278,7 +1278,7 @@ rd_status rd_encode_jpeg(rd_ctx* h, const uint8_t* rgb, uint32_t width, uint32_t
 }
 
 rd_status rd_check_math(rd_ctx* h, int32_t which, uint64_t* result) {
-  if (!h || !result || which < 0 || which > 4) return finish(h, Status{RD_INVALID_INPUT, "bad argument"});
+  if (!h || !result || which < 0 || which > 6) return finish(h, Status{RD_INVALID_INPUT, "bad argument"});
   cudaSetDevice(h->c.device);
   if (which == 4) return finish(h, rd::run_hypot_check(h->c, result));
   return finish(h, rd::run_math_check(h->c, which, result));

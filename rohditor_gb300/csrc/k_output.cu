@@ -570,6 +570,99 @@ __global__ void quantize_check_kernel(unsigned int first, unsigned int last, uns
   if ((threadIdx.x & 31) == 0 && bad) atomicAdd(failures, (unsigned long long)bad);
 }
 
+// quick_div against the IEEE division. Every significand of the divisor, with
+// numerators of two kinds: the hard ones, whose quotient lies next to the middle
+// between two f32 (a 2^s = b t + r for an odd t and the smallest r, found from the
+// inverse of b modulo a power of two), and hashed ones; each pair at exponent 0
+// and at one end of the range. Divisors whose refined reciprocal is not the
+// rounded one go to `list` for quotient_list_check_kernel.
+constexpr int QUOTIENT_NUMERATORS = 4096, QUOTIENT_LIST = 4096;
+__device__ __forceinline__ unsigned hashed(unsigned v) {
+  v *= 2654435761u;
+  v ^= v >> 15;
+  v *= 2246822519u;
+  v ^= v >> 13;
+  return v;
+}
+__device__ __forceinline__ unsigned quotient_differs(unsigned a, unsigned b, unsigned h) {
+  constexpr int PAIRS = 12;
+  const signed char ends[PAIRS][2] = {{99, 0}, {-99, 0}, {0, 99},    {0, -99},     {49, -50}, {-50, 49},
+                                      {99, 99}, {-100, -100}, {-100, -1}, {99, 1}, {60, 60}, {-60, -30}};
+  const int k = (int)(h % PAIRS);
+  const unsigned sign = (h << 3) & 0x80000000u;
+  auto at = [](unsigned significand, int exponent) {
+    return __uint_as_float((significand & 0x7fffffu) | ((unsigned)(exponent + 127) << 23));
+  };
+  unsigned bad = 0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const float x = __uint_as_float(__float_as_uint(at(a, j ? ends[k][0] : 0)) ^ sign), y = at(b, j ? ends[k][1] : 0);
+    bad += __float_as_uint(quick_div(x, y)) != __float_as_uint(__fdiv_rn(x, y));
+  }
+  return bad;
+}
+__global__ void quotient_check_kernel(unsigned long long* failures, unsigned* list) {
+  unsigned long long bad = 0;
+  for (unsigned b = 0x800000u + blockIdx.x * blockDim.x + threadIdx.x; b < 0x1000000u; b += gridDim.x * blockDim.x) {
+    const float divisor = __uint_as_float((b & 0x7fffffu) | 0x3f800000u);
+    if (__float_as_uint(reciprocal_of(divisor)) != __float_as_uint(__fdiv_rn(1.0f, divisor))) {
+      const unsigned at = atomicAdd(list, 1u);
+      if (at < (unsigned)QUOTIENT_LIST) list[1 + at] = b;
+    }
+    const int e = __ffs((int)b) - 1;
+    const unsigned odd = b >> e;
+    unsigned inverse = odd;  // modulo 2^3, then 2^6 .. 2^48
+    for (int k = 0; k < 4; ++k) inverse *= 2u - odd * inverse;
+    unsigned done = 0;
+    for (int k = 0; k < 8; ++k) {
+      const int s = 24 + (k & 1), r = ((k & 2) ? 3 : 1) * ((k & 4) ? -1 : 1);
+      // b t = a 2^s - r 2^e with t in (2^24, 2^25): below 2^e the bits of t are free.
+      unsigned t = (unsigned)(-r) * inverse & ((1u << (s - e)) - 1u);
+      t |= hashed(b + k) << (s - e);
+      t = (t & 0xffffffu) | 0x1000000u;
+      if (s == 25 && e == 0 && !(((unsigned)(-r) * inverse) & 0x1000000u)) continue;
+      const long long n = (long long)b * t + (long long)r * (1ll << e);
+      if (n & ((1ll << s) - 1)) continue;
+      const long long a = n >> s;
+      if (a < 0x800000ll || a > 0xffffffll) continue;
+      bad += quotient_differs((unsigned)a, b, hashed(b * 8u + k));
+      ++done;
+    }
+    for (unsigned k = done; k < (unsigned)QUOTIENT_NUMERATORS; ++k) {
+      const unsigned h = hashed(b * 4096u + k);
+      bad += quotient_differs(h, b, hashed(h));
+    }
+  }
+  if (bad) atomicAdd(failures, bad);
+}
+// Every numerator for the listed divisors; a list that overflowed counts as a failure.
+__global__ void quotient_list_check_kernel(unsigned long long* failures, const unsigned* list) {
+  const unsigned n = min(list[0], (unsigned)QUOTIENT_LIST);
+  unsigned long long bad = blockIdx.x == 0 && threadIdx.x == 0 && list[0] > (unsigned)QUOTIENT_LIST;
+  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < 0x800000u; a += gridDim.x * blockDim.x)
+    for (unsigned k = 0; k < n; ++k) bad += quotient_differs(a, list[1 + k], hashed(a + k));
+  if (bad) atomicAdd(failures, bad);
+}
+// divide_by with the rounded reciprocal of a constant: the listed ones, then the
+// widths between the HSL band centres; every significand at five exponents.
+struct ConstantDivisors {
+  float b[CONSTANT_DIVISOR_COUNT];
+};
+__global__ void constant_quotient_check_kernel(const ConstantDivisors c, unsigned long long* failures) {
+  unsigned long long bad = 0;
+  for (int k = 0; k < CONSTANT_DIVISOR_COUNT + 8; ++k) {
+    const int h = k - CONSTANT_DIVISOR_COUNT;
+    const float b = h < 0 ? c.b[k] : (h == 7 ? 1.0f : HSL_CENTERS[(h + 1) & 7]) - HSL_CENTERS[h & 7];
+    const float y = __fdiv_rn(1.0f, b);
+    for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < 0x800000u; a += gridDim.x * blockDim.x)
+      for (int e = -100; e <= 100; e += 50) {
+        const float x = __uint_as_float(a | ((unsigned)(e + 127) << 23));
+        bad += __float_as_uint(divide_by(x, b, y)) != __float_as_uint(__fdiv_rn(x, b));
+      }
+  }
+  if (bad) atomicAdd(failures, bad);
+}
+
 // Host copy of cbrt_rn's method (std::cbrt in double as the estimate).
 float cbrt_rn_host(float x) {
   if (x == 0.0f || !std::isfinite(x)) return x;
@@ -719,9 +812,11 @@ Status run_display_output(Context& ctx, const float* rgb, const rd_color_desc& c
 }
 
 Status run_math_check(Context& ctx, int which, uint64_t* result) {
+  // The result, then (which 5) the list of divisors.
+  const size_t bytes = 16 + (which == 5 ? sizeof(unsigned) * (1 + QUOTIENT_LIST) : 0);
   void* p = nullptr;
-  RD_TRY(device_alloc(ctx, 16, &p));
-  RD_CUDA_TRY(cudaMemsetAsync(p, 0, 16, ctx.stream));
+  RD_TRY(device_alloc(ctx, bytes, &p));
+  RD_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, ctx.stream));
   const int grid = (ctx.sm_count > 0 ? ctx.sm_count : 152) * 8;
   const float lo = 0.0031308f, one = 1.0f;
   unsigned int first = 0, last = 0;
@@ -735,6 +830,17 @@ Status run_math_check(Context& ctx, int which, uint64_t* result) {
   } else if (which == 2) {
     RD_LAUNCH(ctx, K_OUTPUT, (transfer_rn_check_kernel<<<grid, 256, 0, ctx.stream>>>(
                                  first + 1, last, static_cast<unsigned long long*>(p))));
+  } else if (which == 5) {
+    unsigned* list = static_cast<unsigned*>(p) + 4;
+    RD_LAUNCH(ctx, K_OUTPUT,
+              (quotient_check_kernel<<<grid, 256, 0, ctx.stream>>>(static_cast<unsigned long long*>(p), list)));
+    RD_LAUNCH(ctx, K_OUTPUT,
+              (quotient_list_check_kernel<<<grid, 256, 0, ctx.stream>>>(static_cast<unsigned long long*>(p), list)));
+  } else if (which == 6) {
+    ConstantDivisors c;
+    for (int k = 0; k < CONSTANT_DIVISOR_COUNT; ++k) c.b[k] = CONSTANT_DIVISORS[k];
+    RD_LAUNCH(ctx, K_OUTPUT, (constant_quotient_check_kernel<<<grid, 256, 0, ctx.stream>>>(
+                                 c, static_cast<unsigned long long*>(p))));
   } else {
     RD_LAUNCH(ctx, K_OUTPUT, (quantize_check_kernel<<<grid, 256, 0, ctx.stream>>>(
                                  first + 1, last, static_cast<unsigned long long*>(p))));
@@ -744,7 +850,7 @@ Status run_math_check(Context& ctx, int which, uint64_t* result) {
   if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(&v, p, 8, cudaMemcpyDeviceToHost, ctx.stream) != cudaSuccess ||
       cudaStreamSynchronize(ctx.stream) != cudaSuccess)
     st = Status{RD_SYNCHRONIZATION, "math check failed"};
-  device_free(ctx, p, 16);
+  device_free(ctx, p, bytes);
   if (st.ok()) *result = which == 1 ? (v & 0xffffffffull) : v;
   return st;
 }

@@ -714,7 +714,8 @@ class Stages:
 
     def check_math(self, which: int) -> int:
         """rd_check_math: 0 -> cube roots not correctly rounded; 1 -> the transfer estimate's largest distance in ulps;
-        2, 3 -> transfer powers / quantised codes off the correctly rounded ones; 4 -> optics hypot mismatches."""
+        2, 3 -> transfer powers / quantised codes off the correctly rounded ones; 4 -> optics hypot mismatches;
+        5, 6 -> quotients of the special-case-free division (any divisor, constant ones) off the IEEE ones."""
         v = ctypes.c_uint64()
         self.device.check(self.lib.rd_check_math(self.device.handle, which, ctypes.byref(v)))
         return v.value
