@@ -1390,24 +1390,35 @@ Status rl_prep(Context& ctx, int r, const Taps& taps, const float* rgb, long lon
 // ---- launch-shape tuning of the RL iteration -----------------------------------
 // How many row segments each strip is cut into is a pure scheduling choice:
 // every output of an iteration is computed the same way whatever the
-// segmentation. The first develop of an image shape (width, height, radius)
-// therefore runs iterations 1..K-1 under the candidate segment counts in turn
-// (iteration 0, which may pay for loading the kernel, under the heuristic's
-// count and untimed), each timed with events; after the develop's
-// synchronisation the candidate with the fastest iteration is kept for that
-// shape in a process-wide table, and later develops of the shape use it.
+// segmentation. The first develops of an image shape (width, height, radius)
+// therefore run iterations 1..K-2 under the candidate segment counts in turn,
+// each timed with events (iteration 0 may pay for loading the kernel and the
+// last one also applies the gain; both run under the heuristic's count,
+// untimed). The times are folded into a process-wide table after a develop's
+// synchronisation. Once every candidate has one, which takes one develop of five
+// iterations for three candidates and several of fewer, the fastest is kept for
+// the shape; from two iterations down nothing is timed.
 struct RlShape {
   int W, H, R;
   bool operator<(const RlShape& o) const {
     return W != o.W ? W < o.W : (H != o.H ? H < o.H : R < o.R);
   }
 };
-struct RlChoice {
-  int segs = 0, default_segs = 0;
-  float best_ms = 0.0f, default_ms = 0.0f;
+struct RlTuning {
+  std::vector<int> cands;    // the heuristic's count first
+  std::vector<float> best;   // fastest timed iteration per candidate (ms), < 0 until timed
+  size_t issued = 0;         // timed iterations handed out
+  int segs = 0;              // the choice; 0 until every candidate is timed
 };
 std::mutex g_rl_tune_mutex;
-std::map<RlShape, RlChoice> g_rl_tuned;
+std::map<RlShape, RlTuning> g_rl_tuned;
+
+// The chosen count of a shape, 0 while there is none.
+int rl_tuned_segments(const RlShape& key) {
+  std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
+  const auto it = g_rl_tuned.find(key);
+  return it == g_rl_tuned.end() ? 0 : it->second.segs;
+}
 
 // The occupancy heuristic: one round of (strip, segment) items over all
 // resident warps or CTAs. The strip kernel's segments go down to 8 rows: a small
@@ -1449,32 +1460,25 @@ std::vector<int> rl_candidates(int H, int d) {
 }  // namespace
 
 void resolve_rl_tuning(Context& ctx) {
-  std::map<int, float> best;  // candidate -> fastest timed iteration
+  std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
+  RlTuning& t = g_rl_tuned[RlShape{ctx.tune_shape[0], ctx.tune_shape[1], ctx.tune_shape[2]}];
   for (auto& r : ctx.tune_runs) {
     float ms = 0.0f;
-    if (cudaEventElapsedTime(&ms, r.second.first, r.second.second) == cudaSuccess) {
-      auto it = best.find(r.first);
-      if (it == best.end() || ms < it->second) best[r.first] = ms;
-    }
+    const bool ok = cudaEventElapsedTime(&ms, r.second.first, r.second.second) == cudaSuccess;
     ctx.event_pool.push_back(r.second.first);
     ctx.event_pool.push_back(r.second.second);
+    for (size_t k = 0; ok && t.segs == 0 && k < t.cands.size(); ++k)
+      if (t.cands[k] == r.first && (t.best[k] < 0.0f || ms < t.best[k])) t.best[k] = ms;
   }
   ctx.tune_runs.clear();
   cudaGetLastError();
-  const RlShape key{ctx.tune_shape[0], ctx.tune_shape[1], ctx.tune_shape[2]};
-  const int d = rl_default_segments(key.W, key.H, key.R, ctx.sm_count > 0 ? ctx.sm_count : 152);
-  RlChoice c;
-  c.default_segs = d;
-  for (auto& kv : best) {
-    if (kv.first == d) c.default_ms = kv.second;
-    if (c.segs == 0 || kv.second < c.best_ms) {
-      c.segs = kv.first;
-      c.best_ms = kv.second;
-    }
+  if (t.segs || t.best.empty()) return;
+  size_t fastest = 0;
+  for (size_t k = 0; k < t.best.size(); ++k) {
+    if (t.best[k] < 0.0f) return;
+    if (t.best[k] < t.best[fastest]) fastest = k;
   }
-  if (c.segs == 0) return;
-  std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
-  g_rl_tuned[key] = c;
+  t.segs = t.cands[fastest];
 }
 
 namespace {
@@ -1781,21 +1785,25 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
     // Launch shape: the tuned segment count of this image shape, or a tuning
     // run over the candidates (not while the stream is being captured).
     const RlShape shape{W, H, r};
-    int segs = 0;
-    {
-      std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
-      auto it = g_rl_tuned.find(shape);
-      if (it != g_rl_tuned.end()) segs = it->second.segs;
-    }
+    int segs = rl_tuned_segments(shape);
     std::vector<int> cands;
+    size_t next_cand = 0;
     if (segs == 0) {
       segs = rl_default_segments(W, H, r, ctx.sm_count > 0 ? ctx.sm_count : 152);
-      if (!ctx.capturing && ctx.tune_runs.empty() && detail.iterations >= 3) cands = rl_candidates(H, segs);
-    }
-    if (!cands.empty()) {
-      ctx.tune_shape[0] = W;
-      ctx.tune_shape[1] = H;
-      ctx.tune_shape[2] = r;
+      if (!ctx.capturing && ctx.tune_runs.empty() && detail.iterations >= 3) {
+        ctx.tune_shape[0] = W;
+        ctx.tune_shape[1] = H;
+        ctx.tune_shape[2] = r;
+        std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
+        RlTuning& t = g_rl_tuned[shape];
+        if (t.cands.empty()) {
+          t.cands = rl_candidates(H, segs);
+          t.best.assign(t.cands.size(), -1.0f);
+        }
+        cands = t.cands;
+        next_cand = t.issued;
+        t.issued += (size_t)detail.iterations - 2;
+      }
     }
     for (int it = 0; it < detail.iterations && st.ok(); ++it) {
       // The last iteration of a strip image applies the gain too; it is not
@@ -1805,7 +1813,7 @@ Status run_capture(Context& ctx, float* rgb, int W, int H, const rd_detail_desc&
       if (last && rl_uses_strip_kernel(W, H, r)) gain = GainStep{rgb, mask, detail.amount};
       gained = gain.rgb != nullptr;
       const bool timed = !cands.empty() && it > 0 && !last;
-      const int s_it = timed ? cands[(it - 1) % cands.size()] : segs;
+      const int s_it = timed ? cands[(next_cand + (size_t)(it - 1)) % cands.size()] : segs;
       cudaEvent_t a = nullptr, b = nullptr;
       if (timed) {
         for (cudaEvent_t* e : {&a, &b}) {
@@ -1941,12 +1949,7 @@ Status run_capture_images(Context& ctx, CaptureJob* jobs, int n) {
       continue;
     }
     cp.vec = strip_vector(cp.planes, W) && strip_vector(job.rgb, W);
-    int segs = 0;
-    {
-      std::lock_guard<std::mutex> lk(g_rl_tune_mutex);
-      auto it = g_rl_tuned.find(RlShape{W, H, cp.r});
-      if (it != g_rl_tuned.end()) segs = it->second.segs;
-    }
+    int segs = rl_tuned_segments(RlShape{W, H, cp.r});
     if (segs == 0) segs = rl_default_segments(W, H, cp.r, sms);
     cp.segs = strip_segments(H, segs);
     cp.iterations = d.iterations;
@@ -2049,12 +2052,13 @@ extern "C" rd_status rd_rl_launch_shape(uint32_t width, uint32_t height, float r
   if (taps < 0 || !segments) return RD_INVALID_INPUT;
   const rd::RlShape key{(int)width, (int)height, taps / 2};
   std::lock_guard<std::mutex> lk(rd::g_rl_tune_mutex);
-  auto it = rd::g_rl_tuned.find(key);
-  if (it == rd::g_rl_tuned.end()) return RD_UNSUPPORTED;
-  *segments = it->second.segs;
-  if (default_segments) *default_segments = it->second.default_segs;
-  if (best_ms) *best_ms = it->second.best_ms;
-  if (default_ms) *default_ms = it->second.default_ms;
+  const auto it = rd::g_rl_tuned.find(key);
+  if (it == rd::g_rl_tuned.end() || it->second.segs == 0) return RD_UNSUPPORTED;
+  const rd::RlTuning& t = it->second;
+  *segments = t.segs;
+  if (default_segments) *default_segments = t.cands[0];
+  if (best_ms) *best_ms = *std::min_element(t.best.begin(), t.best.end());
+  if (default_ms) *default_ms = t.best[0];
   return RD_OK;
 }
 

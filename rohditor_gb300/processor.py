@@ -295,8 +295,8 @@ class RlLaunchShape:
 
 
 def rl_launch_shape(width: int, height: int, radius: float) -> RlLaunchShape | None:
-    """rd_rl_launch_shape: the row-segment count the first develop of this
-    (width, height, radius) picked by timing, or None before any develop of it."""
+    """rd_rl_launch_shape: the row-segment count the first develops of this
+    (width, height, radius) picked by timing, or None until they have timed every candidate."""
     segs, dflt = ctypes.c_int32(), ctypes.c_int32()
     best, dms = ctypes.c_float(), ctypes.c_float()
     code = _ffi.load().rd_rl_launch_shape(width, height, radius, ctypes.byref(segs), ctypes.byref(dflt),
