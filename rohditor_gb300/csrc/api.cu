@@ -33,29 +33,39 @@ Status reserve(Context& ctx, size_t bytes) {
 }
 void release(Context& ctx, size_t bytes) { ctx.reserved -= std::min<uint64_t>(bytes, ctx.reserved); }
 
-// Every context's kept blocks can be given back when the device runs out of
-// memory; the registry is what finds them.
-std::mutex g_contexts_mutex;
-std::vector<Context*> g_contexts;
-
-void release_kept_blocks(Context& ctx) {
-  std::lock_guard<std::mutex> lk(ctx.blocks.mutex);
-  for (auto& b : ctx.blocks.kept) cudaFreeAsync(b.first, ctx.stream);
-  ctx.blocks.kept.clear();
-  ctx.blocks.bytes = 0;
+int PoolCalls::malloc_async(void** out, size_t bytes, cudaStream_t s) {
+  const cudaError_t e = cudaMallocAsync(out, bytes, s);
+  if (e != cudaSuccess) cudaGetLastError();
+  return (int)e;
 }
+bool PoolCalls::free_async(void* ptr, cudaStream_t s) {
+  if (cudaFreeAsync(ptr, s) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+void PoolCalls::follow(cudaStream_t waiter, cudaStream_t s) {
+  cudaEvent_t e = nullptr;
+  if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
+    cudaEventRecord(e, s);
+    cudaStreamWaitEvent(waiter, e, 0);
+    cudaEventDestroy(e);
+  }
+  cudaGetLastError();
+}
+void PoolCalls::finish(cudaStream_t s) { cudaStreamSynchronize(s); }
 
 // Pinning memory takes longer than a batch's whole set-up, and a batch makes its
 // contexts anew: up to eight areas (528 KB each) wait here for the next context.
 constexpr size_t SPARE_AREAS = 8;
-std::vector<unsigned char*> g_spare_areas;  // under g_contexts_mutex
+std::mutex g_spare_mutex;
+std::vector<unsigned char*> g_spare_areas;  // under g_spare_mutex
 
 bool take_pinned_area(PinnedArea& a) {
   constexpr size_t bytes = 2 * PinnedArea::HALF + PinnedArea::READBACK;
   for (auto& e : a.done)
     if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) e = nullptr;
   if (a.done[0] && a.done[1]) {
-    std::lock_guard<std::mutex> lk(g_contexts_mutex);
+    std::lock_guard<std::mutex> lk(g_spare_mutex);
     if (!g_spare_areas.empty()) {
       a.base = g_spare_areas.back();
       g_spare_areas.pop_back();
@@ -74,7 +84,7 @@ bool take_pinned_area(PinnedArea& a) {
 // After the last copy into or out of it.
 void give_pinned_area(PinnedArea& a) {
   if (a.pinned) {
-    std::lock_guard<std::mutex> lk(g_contexts_mutex);
+    std::lock_guard<std::mutex> lk(g_spare_mutex);
     if (g_spare_areas.size() < SPARE_AREAS) g_spare_areas.push_back(a.base);
     else cudaFreeHost(a.base);
   } else {
@@ -94,65 +104,26 @@ Status device_alloc(Context& ctx, size_t bytes, void** out) {
   *out = nullptr;
   if (bytes == 0) bytes = 16;
   RD_TRY(reserve(ctx, bytes));
-  BlockCache& cache = ctx.blocks;
-  if (!ctx.capturing) {
-    std::lock_guard<std::mutex> lk(cache.mutex);
-    for (size_t k = cache.kept.size(); k-- > 0;)
-      if (cache.kept[k].second == bytes) {
-        *out = cache.kept[k].first;
-        cache.kept.erase(cache.kept.begin() + (long)k);
-        cache.bytes -= bytes;
-        cache.live[*out] = bytes;
-        return Status{};
-      }
-  }
-  cudaError_t e = cudaMallocAsync(out, bytes, ctx.stream);
-  if (e != cudaSuccess && !ctx.capturing) {
-    cudaGetLastError();
-    {
-      std::lock_guard<std::mutex> lk(g_contexts_mutex);
-      for (Context* c : g_contexts)
-        if (c->device == ctx.device && !c->capturing) {
-          release_kept_blocks(*c);
-          cudaStreamSynchronize(c->stream);
-        }
-    }
-    e = cudaMallocAsync(out, bytes, ctx.stream);
-  }
-  if (e != cudaSuccess) {
+  const int e = ctx.capturing ? PoolCalls::malloc_async(out, bytes, ctx.stream) : ctx.blocks.alloc(bytes, out);
+  if (e) {
     release(ctx, bytes);
-    cudaGetLastError();
-    return Status{RD_OVER_BUDGET, std::string("device allocation failed: ") + cudaGetErrorString(e)};
-  }
-  if (!ctx.capturing) {
-    std::lock_guard<std::mutex> lk(cache.mutex);
-    cache.live[*out] = bytes;
+    return Status{RD_OVER_BUDGET, std::string("device allocation failed: ") + cudaGetErrorString((cudaError_t)e)};
   }
   return Status{};
 }
 void device_free(Context& ctx, void* ptr, size_t bytes) {
   if (!ptr) return;
   release(ctx, bytes == 0 ? 16 : bytes);
-  {
-    BlockCache& cache = ctx.blocks;
-    std::lock_guard<std::mutex> lk(cache.mutex);
-    const auto it = cache.live.find(ptr);
-    if (it != cache.live.end()) {
-      const size_t size = it->second;
-      cache.live.erase(it);
-      if (!ctx.capturing && size <= BLOCK_CACHE_BYTES) {
-        cache.kept.emplace_back(ptr, size);
-        cache.bytes += size;
-        while (cache.bytes > BLOCK_CACHE_BYTES || cache.kept.size() > BLOCK_CACHE_BLOCKS) {
-          cudaFreeAsync(cache.kept.front().first, ctx.stream);
-          cache.bytes -= cache.kept.front().second;
-          cache.kept.erase(cache.kept.begin());
-        }
-        return;
-      }
-    }
-  }
-  cudaFreeAsync(ptr, ctx.stream);
+  ctx.blocks.free(ptr);
+}
+
+void begin_capture(Context& ctx) {
+  ctx.blocks.close();
+  ctx.capturing = true;
+}
+void end_capture(Context& ctx) {
+  ctx.capturing = false;
+  ctx.blocks.open();
 }
 
 const char* kernel_family_name(int family) {
@@ -209,8 +180,10 @@ Status set_stream_priority(Context& c, bool high) {
   RD_CUDA_TRY(cudaStreamSynchronize(c.stream));
   cudaStream_t s = nullptr;
   RD_CUDA_TRY(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, high ? greatest : least));
-  cudaStreamDestroy(c.stream);
-  c.stream = s;
+  c.blocks.replace_stream([&] {
+    cudaStreamDestroy(c.stream);
+    return c.stream = s;
+  });
   return Status{};
 }
 
@@ -222,7 +195,7 @@ Status upload(Context& ctx, void* dst, const void* src, size_t bytes) {
   if (!ctx.capturing) {
     PinnedArea& area = ctx.pinned;
     if (area.pinned && bytes <= PinnedArea::HALF) {
-      std::lock_guard<std::mutex> lk(ctx.blocks.mutex);
+      std::lock_guard<std::mutex> lk(ctx.pinned_mutex);
       bool room = area.used + bytes <= PinnedArea::HALF;
       if (!room) {
         const int other = area.half ^ 1;
@@ -743,10 +716,7 @@ rd_status rd_ctx_create(int device, uint64_t budget_bytes, rd_ctx** out) {
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
   }
   cudaStreamSynchronize(c.stream);
-  {
-    std::lock_guard<std::mutex> lk(rd::g_contexts_mutex);
-    rd::g_contexts.push_back(&c);
-  }
+  c.blocks.attach(device, c.stream);
   *out = h;
   return RD_OK;
 }
@@ -758,11 +728,7 @@ void rd_ctx_destroy(rd_ctx* h) {
   cudaSetDevice(c.device);
   if (c.amaze_scratch) rd::device_free(c, c.amaze_scratch, c.amaze_bytes);
   if (c.flush_buf) rd::device_free(c, c.flush_buf, c.flush_bytes);
-  {
-    std::lock_guard<std::mutex> lk(rd::g_contexts_mutex);
-    rd::g_contexts.erase(std::find(rd::g_contexts.begin(), rd::g_contexts.end(), &c));
-  }
-  rd::release_kept_blocks(c);
+  c.blocks.detach();
   cudaStreamSynchronize(c.stream);
   for (void* p : c.pinned_uploads) cudaFreeHost(p);
   rd::give_pinned_area(c.pinned);
@@ -2034,8 +2000,8 @@ extern "C" rd_status rd_develop_batch_flat_graph(int device, rd_batch_item* item
         cudaEventRecord(fork, main) != cudaSuccess)
       status = RD_SYNCHRONIZATION;
     for (int c = 0; c < chains && status == RD_OK; ++c) {
+      rd::begin_capture(ctxs[c]->c);
       if (cudaStreamWaitEvent(ctxs[c]->c.stream, fork, 0) != cudaSuccess) status = RD_SYNCHRONIZATION;
-      ctxs[c]->c.capturing = true;
     }
     // 1. upload + normalize + highlight on the branches.
     for (int k = 0; k < count && status == RD_OK; ++k) {
@@ -2091,13 +2057,12 @@ extern "C" rd_status rd_develop_batch_flat_graph(int device, rd_batch_item* item
       if (base) rd_base_release(base);
       if (st != RD_OK) status = st;
     }
-    for (int c = 0; c < chains; ++c) {
-      ctxs[c]->c.capturing = false;
+    for (int c = 0; c < chains; ++c)
       if (cudaEventRecord(join[c], ctxs[c]->c.stream) != cudaSuccess ||
           cudaStreamWaitEvent(main, join[c], 0) != cudaSuccess)
         if (status == RD_OK) status = RD_SYNCHRONIZATION;
-    }
     const cudaError_t end = cudaStreamEndCapture(main, &graph);
+    for (int c = 0; c < chains; ++c) rd::end_capture(ctxs[c]->c);
     if (end != cudaSuccess && status == RD_OK) status = RD_SYNCHRONIZATION;
     if (status == RD_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) status = RD_SYNCHRONIZATION;
     cudaGetLastError();

@@ -138,8 +138,8 @@ extern "C" rd_status rd_develop_batch_graph(int device, rd_batch_item* items, in
         cudaEventRecord(fork, main) != cudaSuccess)
       status = RD_SYNCHRONIZATION;
     for (int c = 0; c < chains && status == RD_OK; ++c) {
+      rd::begin_capture(ctxs[c]->c);
       if (cudaStreamWaitEvent(ctxs[c]->c.stream, fork, 0) != cudaSuccess) status = RD_SYNCHRONIZATION;
-      ctxs[c]->c.capturing = true;
     }
     for (int k = 0; k < count && status == RD_OK; ++k) {
       rd_batch_item& it = items[k];
@@ -157,13 +157,12 @@ extern "C" rd_status rd_develop_batch_graph(int device, rd_batch_item* items, in
       if (base) rd_base_release(base);
       if (st != RD_OK) status = st;
     }
-    for (int c = 0; c < chains; ++c) {
-      ctxs[c]->c.capturing = false;
+    for (int c = 0; c < chains; ++c)
       if (cudaEventRecord(join[c], ctxs[c]->c.stream) != cudaSuccess ||
           cudaStreamWaitEvent(main, join[c], 0) != cudaSuccess)
         if (status == RD_OK) status = RD_SYNCHRONIZATION;
-    }
     const cudaError_t end = cudaStreamEndCapture(main, &graph);
+    for (int c = 0; c < chains; ++c) rd::end_capture(ctxs[c]->c);
     if (end != cudaSuccess && status == RD_OK) status = RD_SYNCHRONIZATION;
     if (status == RD_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) status = RD_SYNCHRONIZATION;
     cudaGetLastError();

@@ -17,6 +17,7 @@
 
 #include "../../include/rd_gpu.h"
 
+#include "block_cache.cuh"
 #include "quick_div.cuh"
 
 namespace rd {
@@ -66,16 +67,14 @@ struct ShapePick {
   int value = 0;
   cudaEvent_t start = nullptr;  // set when this launch is timed
 };
-// Device blocks that a context has freed and keeps for its next allocation of
-// the same size, oldest first, and the sizes of those it has handed out.
-struct BlockCache {
-  std::mutex mutex;
-  std::vector<std::pair<void*, size_t>> kept;
-  std::unordered_map<void*, size_t> live;
-  size_t bytes = 0;  // of the kept blocks
+// The pool calls of a context's kept blocks (block_cache.cuh).
+struct PoolCalls {
+  using Stream = cudaStream_t;
+  static int malloc_async(void** out, size_t bytes, cudaStream_t s);
+  static bool free_async(void* ptr, cudaStream_t s);
+  static void follow(cudaStream_t waiter, cudaStream_t s);
+  static void finish(cudaStream_t s);
 };
-constexpr size_t BLOCK_CACHE_BYTES = size_t(8) << 30;
-constexpr size_t BLOCK_CACHE_BLOCKS = 64;
 
 // Pinned host memory of a context: two halves that small uploads go through in
 // turn, and a place for what a call reads back.
@@ -129,8 +128,9 @@ struct Context {
   // one item.
   bool yield_sms = false;
   std::vector<void*> pinned_uploads;
-  BlockCache blocks;
+  BlockCache<PoolCalls> blocks;
   PinnedArea pinned;
+  std::mutex pinned_mutex;  // of the upload halves
   // Timed RL iterations of a launch-shape tuning run, resolved after the
   // stage's synchronisation: (candidate segment count, start, end).
   int tune_shape[3] = {0, 0, 0};
@@ -203,6 +203,10 @@ Status device_alloc(Context& ctx, size_t bytes, void** out);
 void device_free(Context& ctx, void* ptr, size_t bytes);
 Status check_kernel_error(Context& ctx, const char* stage);
 Status set_stream_priority(Context& ctx, bool high);
+// Around a stream capture that the context's stream is to join: before it does,
+// and after the capture has ended.
+void begin_capture(Context& ctx);
+void end_capture(Context& ctx);
 
 // ------------------------------------------------------------------ mosaic source
 // Per-sample view of the (cropped, normalized, highlight-processed) mosaic,
