@@ -158,7 +158,17 @@ typedef struct rd_metrics {
 rd_status rd_ctx_create(int device, uint64_t budget_bytes, rd_ctx** out);
 /* Every rd_source and rd_base of the context must be released first. */
 void rd_ctx_destroy(rd_ctx* ctx);
+/* A context keeps device blocks that it has freed for its next calls; what it
+ * holds and what it keeps stay within the budget together (0: no budget; up to
+ * 8 GiB are kept). Lowering the budget gives the excess back. */
 rd_status rd_ctx_set_budget(rd_ctx* ctx, uint64_t budget_bytes);
+/* Bytes that the context keeps for its next calls. Kept blocks are given back
+ * when an allocation of any context of the device fails; a program that needs
+ * the memory for something else gives them back with rd_ctx_trim. */
+uint64_t rd_ctx_kept_bytes(const rd_ctx* ctx);
+/* Gives kept blocks back until no more than `keep_bytes` are kept, waits for the
+ * context's work and returns the pool's unused memory to the device. */
+rd_status rd_ctx_trim(rd_ctx* ctx, uint64_t keep_bytes);
 const char* rd_ctx_last_error(const rd_ctx* ctx);
 rd_status rd_ctx_synchronize(rd_ctx* ctx);
 /* Number of this library's kernels launched on the context so far. */

@@ -162,6 +162,8 @@ SIGNATURES = {
     "rd_ctx_create": (ctypes.c_int, [ctypes.c_int, ctypes.c_uint64, ctypes.POINTER(VOIDP)]),
     "rd_ctx_destroy": (None, [VOIDP]),
     "rd_ctx_set_budget": (ctypes.c_int, [VOIDP, ctypes.c_uint64]),
+    "rd_ctx_kept_bytes": (ctypes.c_uint64, [VOIDP]),
+    "rd_ctx_trim": (ctypes.c_int, [VOIDP, ctypes.c_uint64]),
     "rd_ctx_last_error": (ctypes.c_char_p, [VOIDP]),
     "rd_ctx_synchronize": (ctypes.c_int, [VOIDP]),
     "rd_ctx_kernel_launches": (ctypes.c_uint64, [VOIDP]),

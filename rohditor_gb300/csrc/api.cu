@@ -1,7 +1,7 @@
 // The C ABI (include/rd_gpu.h): context, processor API, stage entry points and
 // host contract helpers. Everything device-side is ordered on the context's
 // stream; device memory comes from the stream-ordered pool (cudaMallocAsync),
-// in blocks that the context keeps from call to call,
+// in blocks that the context keeps from call to call (block_cache.cuh),
 // and is charged against the context's byte budget before it is taken, like
 // the reference's logical reservations (crates/gpu/src/memory.rs:44-60).
 #include <cuda_runtime.h>
@@ -100,11 +100,21 @@ void give_pinned_area(PinnedArea& a) {
 // blocks have the sizes of the last call's, so the next takes them as they are.
 // A kept block is reused in the order of the context's stream, like one that
 // the pool hands out again. Under stream capture the pool is asked directly.
+// Bytes that the context may keep beside what it holds.
+static size_t keep_room(const Context& ctx) {
+  const uint64_t all = BLOCK_CACHE_BYTES;
+  if (ctx.footprint == 0) return (size_t)all;
+  return (size_t)std::min(all, ctx.footprint - std::min(ctx.footprint, ctx.reserved));
+}
+void trim_kept_blocks(Context& ctx, uint64_t bytes) {
+  ctx.blocks.shrink((size_t)std::min<uint64_t>(bytes, keep_room(ctx)));
+}
+
 Status device_alloc(Context& ctx, size_t bytes, void** out) {
   *out = nullptr;
   if (bytes == 0) bytes = 16;
   RD_TRY(reserve(ctx, bytes));
-  const int e = ctx.capturing ? PoolCalls::malloc_async(out, bytes, ctx.stream) : ctx.blocks.alloc(bytes, out);
+  const int e = ctx.capturing ? PoolCalls::malloc_async(out, bytes, ctx.stream) : ctx.blocks.alloc(bytes, keep_room(ctx), out);
   if (e) {
     release(ctx, bytes);
     return Status{RD_OVER_BUDGET, std::string("device allocation failed: ") + cudaGetErrorString((cudaError_t)e)};
@@ -114,7 +124,7 @@ Status device_alloc(Context& ctx, size_t bytes, void** out) {
 void device_free(Context& ctx, void* ptr, size_t bytes) {
   if (!ptr) return;
   release(ctx, bytes == 0 ? 16 : bytes);
-  ctx.blocks.free(ptr);
+  ctx.blocks.free(ptr, keep_room(ctx));
 }
 
 void begin_capture(Context& ctx) {
@@ -689,7 +699,7 @@ rd_status rd_ctx_create(int device, uint64_t budget_bytes, rd_ctx** out) {
   if (!h) return RD_OVER_BUDGET;
   rd::Context& c = h->c;
   c.device = device;
-  c.budget = budget_bytes;
+  c.budget = c.footprint = budget_bytes;
   cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, device);
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete h;
@@ -752,7 +762,26 @@ void rd_ctx_destroy(rd_ctx* h) {
 
 rd_status rd_ctx_set_budget(rd_ctx* h, uint64_t budget_bytes) {
   if (!h) return RD_INVALID_INPUT;
-  h->c.budget = budget_bytes;
+  rd::Context& c = h->c;
+  c.budget = c.footprint = budget_bytes;
+  cudaSetDevice(c.device);
+  rd::trim_kept_blocks(c, UINT64_MAX);
+  return RD_OK;
+}
+
+uint64_t rd_ctx_kept_bytes(const rd_ctx* h) { return h ? h->c.blocks.kept_bytes() : 0; }
+
+rd_status rd_ctx_trim(rd_ctx* h, uint64_t keep_bytes) {
+  if (!h) return RD_INVALID_INPUT;
+  rd::Context& c = h->c;
+  cudaSetDevice(c.device);
+  rd::trim_kept_blocks(c, keep_bytes);
+  cudaMemPool_t pool = nullptr;
+  if (cudaStreamSynchronize(c.stream) != cudaSuccess || cudaDeviceGetDefaultMemPool(&pool, c.device) != cudaSuccess ||
+      cudaMemPoolTrimTo(pool, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return finish(h, Status{RD_SYNCHRONIZATION, "the pool's memory could not be given back"});
+  }
   return RD_OK;
 }
 

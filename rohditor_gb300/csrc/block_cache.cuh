@@ -2,6 +2,11 @@
 // the same size, and the way they are given back when the device runs out of
 // memory.
 //
+// What is kept is bounded: by the room that the owner names with each call (its
+// budget less what it has in use), by BLOCK_CACHE_BYTES, and by use, since a block
+// that the next BLOCK_CACHE_FREES frees have passed by goes back (a session that
+// opens frames of other sizes does not hold the old sizes' blocks for good).
+//
 // A cache belongs to one context and one thread at a time, its owner, who
 // allocates and frees through it. Any thread whose allocation fails may take the
 // kept blocks of every cache of the device (reclaim). What both touch (the kept
@@ -30,6 +35,7 @@ namespace rd {
 
 constexpr size_t BLOCK_CACHE_BYTES = size_t(8) << 30;
 constexpr size_t BLOCK_CACHE_BLOCKS = 64;
+constexpr uint64_t BLOCK_CACHE_FREES = 256;  // a dozen develops
 
 template <class Gpu>
 class BlockCache {
@@ -65,9 +71,10 @@ class BlockCache {
     shrink(0);
   }
 
-  // Owner: a block of `bytes`, kept or new. When the pool has none, every cache's
-  // kept blocks are given back and it is asked again. 0, or the pool's error.
-  int alloc(size_t bytes, void** out) {
+  // Owner: a block of `bytes`, kept or new; no more than `room` bytes stay kept
+  // beside it. When the pool has none, every cache's kept blocks are given back and
+  // it is asked again. 0, or the pool's error.
+  int alloc(size_t bytes, size_t room, void** out) {
     {
       std::lock_guard<std::mutex> lk(mutex_);
       for (size_t k = kept_.size(); k-- > 0;)
@@ -76,8 +83,10 @@ class BlockCache {
           kept_.erase(kept_.begin() + (ptrdiff_t)k);
           bytes_ -= bytes;
           hand_out(*out, bytes);
+          give_back(room, BLOCK_CACHE_BLOCKS);
           return 0;
         }
+      give_back(room, BLOCK_CACHE_BLOCKS);
     }
     int e = Gpu::malloc_async(out, bytes, stream_);
     if (e) {
@@ -91,20 +100,20 @@ class BlockCache {
     return e;
   }
 
-  // Owner: a block that alloc gave, to be kept; one that it did not give, or any
-  // while the cache is closed, goes back to the pool.
-  void free(void* ptr) {
+  // Owner: a block that alloc gave, to be kept where `room` bytes hold it; one that
+  // it did not give, or any while the cache is closed, goes back to the pool.
+  void free(void* ptr, size_t room) {
     std::lock_guard<std::mutex> lk(mutex_);
     const auto it = live_.find(ptr);
     const size_t bytes = it == live_.end() ? 0 : it->second;
     if (bytes) live_.erase(it);
-    if (bytes == 0 || closed_ || bytes > BLOCK_CACHE_BYTES || kept_.size() == kept_.capacity()) {
+    if (bytes == 0 || closed_ || bytes > room || bytes > BLOCK_CACHE_BYTES || kept_.size() == kept_.capacity()) {
       Gpu::free_async(ptr, stream_);
       return;
     }
-    kept_.push_back(Kept{ptr, bytes});
+    kept_.push_back(Kept{ptr, bytes, ++frees_});
     bytes_ += bytes;
-    give_back(BLOCK_CACHE_BYTES, BLOCK_CACHE_BLOCKS);
+    give_back(room < BLOCK_CACHE_BYTES ? room : BLOCK_CACHE_BYTES, BLOCK_CACHE_BLOCKS);
   }
 
   // Owner: before the stream joins a capture, and after the capture has ended.
@@ -154,6 +163,7 @@ class BlockCache {
   struct Kept {
     void* ptr;
     size_t bytes;
+    uint64_t at;  // the free that brought it
   };
   struct Registry {
     std::mutex mutex;
@@ -171,9 +181,11 @@ class BlockCache {
     } catch (...) {
     }
   }
-  // Under the lock: the oldest first. A block that the pool refuses stays.
+  // Under the lock: the oldest first, down to so many bytes and blocks, and those
+  // that were passed by. A block that the pool refuses stays.
   void give_back(size_t bytes, size_t blocks) {
-    while (!kept_.empty() && (bytes_ > bytes || kept_.size() > blocks)) {
+    while (!kept_.empty() &&
+           (bytes_ > bytes || kept_.size() > blocks || kept_.front().at + BLOCK_CACHE_FREES < frees_)) {
       if (!Gpu::free_async(kept_.front().ptr, stream_)) return;
       bytes_ -= kept_.front().bytes;
       kept_.erase(kept_.begin());
@@ -184,6 +196,7 @@ class BlockCache {
   std::vector<Kept> kept_;                     // oldest first
   std::unordered_map<void*, size_t> live_;     // blocks handed out
   size_t bytes_ = 0;                           // of the kept blocks
+  uint64_t frees_ = 0;                         // blocks kept so far
   bool closed_ = false;
   Stream stream_{};                            // changed by the owner only, under the lock
   int device_ = 0;

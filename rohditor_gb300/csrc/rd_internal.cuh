@@ -93,6 +93,10 @@ struct Context {
   cudaStream_t stream = nullptr;
   uint64_t budget = 0;     // 0 = unlimited
   uint64_t reserved = 0;   // bytes currently held by this context
+  // Bytes that what is held and what is kept for the next calls stay within
+  // together (0: the kept blocks' own limit alone): the budget, or that of the
+  // server whose context it is.
+  uint64_t footprint = 0;
   uint64_t launches = 0;   // kernels launched by this library on this context
   std::string last_error;
   // Error word written by kernels (bounds/footprint/non-finite), read after a stage.
@@ -203,6 +207,9 @@ Status device_alloc(Context& ctx, size_t bytes, void** out);
 void device_free(Context& ctx, void* ptr, size_t bytes);
 Status check_kernel_error(Context& ctx, const char* stage);
 Status set_stream_priority(Context& ctx, bool high);
+// Gives kept blocks back until the context's footprint holds and no more than
+// `bytes` are kept.
+void trim_kept_blocks(Context& ctx, uint64_t bytes);
 // Around a stream capture that the context's stream is to join: before it does,
 // and after the capture has ended.
 void begin_capture(Context& ctx);

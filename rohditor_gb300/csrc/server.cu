@@ -182,9 +182,12 @@ class CudaExecutor : public Executor {
   void* h_stage = nullptr;
   int stage_cap = 0;
 
-  Status init(int device) {
+  Status init(int device, uint64_t budget) {
     RD_TRY(from_code(rd_ctx_create(device, 0, &dev), "develop context"));
     RD_TRY(from_code(rd_ctx_create(device, 0, &ren), "render context"));
+    // What evicted layers and a develop's working set leave behind stays within
+    // the admission budget too.
+    dev->c.footprint = ren->c.footprint = budget;
     RD_TRY(set_stream_priority(dev->c, false));
     dev->c.yield_sms = true;  // renders get SMs within one demosaic work item
     return set_stream_priority(ren->c, true);
@@ -758,7 +761,7 @@ rd_status rd_server_create(int device, uint64_t budget_bytes, rd_server** out) {
   } else {
     // The server does its own admission; the contexts' budgets are left open.
     auto cu = std::make_unique<rd::CudaExecutor>();
-    const rd::Status st = cu->init(device);
+    const rd::Status st = cu->init(device, budget_bytes);
     if (!st.ok()) {
       delete s;
       return st.code;

@@ -365,6 +365,15 @@ class Device:
     def set_budget(self, budget_bytes: int):
         self.check(self.lib.rd_ctx_set_budget(self.handle, budget_bytes))
 
+    @property
+    def kept_bytes(self) -> int:
+        """Device bytes kept for the next calls, beside what is in use."""
+        return int(self.lib.rd_ctx_kept_bytes(self.handle))
+
+    def trim(self, keep_bytes: int = 0):
+        """Gives kept device memory back until at most `keep_bytes` are kept."""
+        self.check(self.lib.rd_ctx_trim(self.handle, keep_bytes))
+
     def synchronize(self):
         self.check(self.lib.rd_ctx_synchronize(self.handle))
 

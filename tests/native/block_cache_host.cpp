@@ -71,6 +71,7 @@ struct FakeGpu {
   }
 };
 using Cache = rd::BlockCache<FakeGpu>;
+constexpr size_t ROOM = ~size_t(0);
 
 void set(FakeStream& s, bool alive, bool capturing) {
   std::lock_guard<std::mutex> lk(g_pool.mutex);
@@ -94,18 +95,18 @@ void reclaim() {
   b.attach(0, &sb);
   other_device.attach(1, &sc);
   void *p = nullptr, *q = nullptr, *r = nullptr;
-  expect(b.alloc(60, &p) == 0 && other_device.alloc(20, &r) == 0, "room at first");
-  b.free(p);
-  other_device.free(r);
+  expect(b.alloc(60, ROOM, &p) == 0 && other_device.alloc(20, ROOM, &r) == 0, "room at first");
+  b.free(p, ROOM);
+  other_device.free(r, ROOM);
   expect(b.kept_bytes() == 60 && other_device.kept_bytes() == 20, "both keep their blocks");
-  expect(a.alloc(70, &q) == 0, "the kept blocks make room");
+  expect(a.alloc(70, ROOM, &q) == 0, "the kept blocks make room");
   expect(b.kept_bytes() == 0 && other_device.kept_bytes() == 20, "of this device only");
   void* none = nullptr;
-  expect(a.alloc(1000, &none) != 0, "more than there is stays refused");
-  a.free(q);
+  expect(a.alloc(1000, ROOM, &none) != 0, "more than there is stays refused");
+  a.free(q, ROOM);
   void* same = nullptr;
-  expect(a.alloc(70, &same) == 0 && same == q, "a kept block serves its size");
-  a.free(same);
+  expect(a.alloc(70, ROOM, &same) == 0 && same == q, "a kept block serves its size");
+  a.free(same, ROOM);
   a.detach();
   b.detach();
   other_device.detach();
@@ -120,18 +121,18 @@ void captured() {
   a.attach(0, &sa);
   b.attach(0, &sb);
   void* p = nullptr;
-  expect(b.alloc(60, &p) == 0, "room");
-  b.free(p);
+  expect(b.alloc(60, ROOM, &p) == 0, "room");
+  b.free(p, ROOM);
   b.close();
   set(sb, true, true);
   void* q = nullptr;
-  expect(a.alloc(70, &q) != 0 && b.kept_bytes() == 60, "its blocks stay");
+  expect(a.alloc(70, ROOM, &q) != 0 && b.kept_bytes() == 60, "its blocks stay");
   b.shrink(0);
   expect(b.kept_bytes() == 60, "and nobody frees into the capture");
   set(sb, true, false);
   b.open();
-  expect(a.alloc(70, &q) == 0 && b.kept_bytes() == 0, "after it they go");
-  a.free(q);
+  expect(a.alloc(70, ROOM, &q) == 0 && b.kept_bytes() == 0, "after it they go");
+  a.free(q, ROOM);
   a.detach();
   b.detach();
   expect(g_pool.in_use == 0, "everything is given back");
@@ -143,13 +144,53 @@ void refused() {
   Cache c;
   c.attach(0, &s);
   void* p[2] = {};
-  for (void*& q : p) expect(c.alloc(10, &q) == 0, "room");
-  for (void* q : p) c.free(q);
+  for (void*& q : p) expect(c.alloc(10, ROOM, &q) == 0, "room");
+  for (void* q : p) c.free(q, ROOM);
   g_pool.refuse_frees = 1;
   c.shrink(0);
   expect(c.kept_bytes() == 20, "refused blocks stay kept");
   c.shrink(0);
   expect(c.kept_bytes() == 0, "and go the next time");
+  c.detach();
+  expect(g_pool.in_use == 0, "everything is given back");
+}
+
+// What is kept stays within the room that a call names, the oldest going first.
+void room() {
+  FakeStream s;
+  Cache c;
+  c.attach(0, &s);
+  void *p[4] = {}, *q = nullptr;
+  for (int k = 0; k < 4; ++k) expect(c.alloc(10 + k, ROOM, &p[k]) == 0, "room");
+  c.free(p[0], 46 - 36);
+  expect(c.kept_bytes() == 10, "what fits is kept");
+  c.free(p[1], 46 - 25);
+  expect(c.kept_bytes() == 21, "both fit");
+  expect(c.alloc(20, 46 - 45, &q) == 0 && c.kept_bytes() == 0, "kept blocks make way for a new one");
+  c.free(q, 10);
+  expect(c.kept_bytes() == 0, "a block larger than the room is not kept");
+  c.free(p[2], ROOM);
+  c.free(p[3], ROOM);
+  c.shrink(13);
+  expect(c.kept_bytes() == 13, "the oldest goes first");
+  c.detach();
+  expect(g_pool.in_use == 0, "everything is given back");
+}
+
+// A block that many frees have passed by goes back.
+void passed_by() {
+  FakeStream s;
+  Cache c;
+  c.attach(0, &s);
+  void* p = nullptr;
+  expect(c.alloc(7, ROOM, &p) == 0, "room");
+  c.free(p, ROOM);
+  for (uint64_t k = 0; k <= rd::BLOCK_CACHE_FREES; ++k) {
+    expect(c.kept_bytes() == (k == 0 ? 7u : 12u), "kept until then");
+    expect(c.alloc(5, ROOM, &p) == 0, "room");
+    c.free(p, ROOM);
+  }
+  expect(c.kept_bytes() == 5, "then it goes");
   c.detach();
   expect(g_pool.in_use == 0, "everything is given back");
 }
@@ -172,7 +213,7 @@ void threads() {
         for (int k = 0; k < 60; ++k) {
           h = h * 1664525u + 1013904223u;
           void* p = nullptr;
-          if (c.alloc(10 + (h >> 24) % 8, &p) == 0) c.free(p);
+          if (c.alloc(10 + (h >> 24) % 8, ROOM, &p) == 0) c.free(p, ROOM);
           if (k % 16 == 5) {
             c.close();
             set(*s, true, true);
@@ -201,7 +242,7 @@ void threads() {
     c.attach(0, &s);
     while (!stop) {
       void* p = nullptr;
-      if (c.alloc(1 << 20, &p) == 0) std::abort();
+      if (c.alloc(1 << 20, ROOM, &p) == 0) std::abort();
       std::this_thread::yield();
     }
     c.detach();
@@ -217,7 +258,8 @@ void threads() {
 
 int main(int argc, char** argv) {
   const std::map<std::string, void (*)()> scenarios = {
-      {"reclaim", reclaim}, {"captured", captured}, {"refused", refused}, {"threads", threads}};
+      {"reclaim", reclaim}, {"captured", captured},   {"refused", refused},
+      {"room", room},       {"passed_by", passed_by}, {"threads", threads}};
   const auto it = argc == 2 ? scenarios.find(argv[1]) : scenarios.end();
   if (it == scenarios.end()) return 2;
   it->second();

@@ -20,7 +20,7 @@ def build(path, *flags):
                           capture_output=True, text=True)
 
 
-@pytest.mark.parametrize("scenario", ["reclaim", "captured", "refused", "threads"])
+@pytest.mark.parametrize("scenario", ["reclaim", "captured", "refused", "room", "passed_by", "threads"])
 def test_kept_blocks(tmp_path, scenario):
     exe = tmp_path / "block_cache_host"
     done = build(exe)
