@@ -127,6 +127,26 @@ void device_free(Context& ctx, void* ptr, size_t bytes) {
   ctx.blocks.free(ptr, keep_room(ctx));
 }
 
+// Calls that take device memory without device_alloc (a graph's memory nodes, a
+// context's error word): once more after every kept block has gone back.
+template <class Call>
+static cudaError_t with_kept_blocks_back(int device, cudaStream_t stream, Call&& call) {
+  cudaError_t e = call();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  BlockCache<PoolCalls>::reclaim(device, stream);
+  cudaMemPool_t pool = nullptr;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+  cudaGetLastError();
+  return call();
+}
+cudaError_t instantiate_graph(int device, cudaGraphExec_t* exec, cudaGraph_t graph, cudaStream_t stream) {
+  return with_kept_blocks_back(device, stream, [&] { return cudaGraphInstantiate(exec, graph, 0); });
+}
+cudaError_t launch_graph(int device, cudaGraphExec_t exec, cudaStream_t stream) {
+  return with_kept_blocks_back(device, stream, [&] { return cudaGraphLaunch(exec, stream); });
+}
+
 void begin_capture(Context& ctx) {
   ctx.blocks.close();
   ctx.capturing = true;
@@ -706,7 +726,8 @@ rd_status rd_ctx_create(int device, uint64_t budget_bytes, rd_ctx** out) {
     return RD_SYNCHRONIZATION;
   }
   for (auto& e : c.ev) cudaEventCreate(&e);
-  if (cudaMalloc(&c.d_error, 4 * sizeof(uint32_t)) != cudaSuccess ||
+  if (rd::with_kept_blocks_back(device, c.stream, [&] { return cudaMalloc(&c.d_error, 4 * sizeof(uint32_t)); }) !=
+          cudaSuccess ||
       cudaMemsetAsync(c.d_error, 0, 4 * sizeof(uint32_t), c.stream) != cudaSuccess) {
     cudaStreamDestroy(c.stream);
     delete h;
@@ -2093,7 +2114,7 @@ extern "C" rd_status rd_develop_batch_flat_graph(int device, rd_batch_item* item
     const cudaError_t end = cudaStreamEndCapture(main, &graph);
     for (int c = 0; c < chains; ++c) rd::end_capture(ctxs[c]->c);
     if (end != cudaSuccess && status == RD_OK) status = RD_SYNCHRONIZATION;
-    if (status == RD_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) status = RD_SYNCHRONIZATION;
+    if (status == RD_OK && rd::instantiate_graph(device, &exec, graph, main) != cudaSuccess) status = RD_SYNCHRONIZATION;
     cudaGetLastError();
   }
   const auto c1 = Clock::now();
@@ -2105,7 +2126,7 @@ extern "C" rd_status rd_develop_batch_flat_graph(int device, rd_batch_item* item
       std::memcpy(stage + in_off[k], it.mosaic, sizeof(uint16_t) * it.row_stride * it.sensor.sensor_height);
     }
     const auto l0 = Clock::now();
-    if (cudaGraphLaunch(exec, main) != cudaSuccess || cudaStreamSynchronize(main) != cudaSuccess)
+    if (rd::launch_graph(device, exec, main) != cudaSuccess || cudaStreamSynchronize(main) != cudaSuccess)
       status = RD_SYNCHRONIZATION;
     if (launch_ms) *launch_ms = std::chrono::duration<double, std::milli>(Clock::now() - l0).count();
     for (int c = 0; c < chains && status == RD_OK; ++c) {

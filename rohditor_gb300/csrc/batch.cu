@@ -164,7 +164,7 @@ extern "C" rd_status rd_develop_batch_graph(int device, rd_batch_item* items, in
     const cudaError_t end = cudaStreamEndCapture(main, &graph);
     for (int c = 0; c < chains; ++c) rd::end_capture(ctxs[c]->c);
     if (end != cudaSuccess && status == RD_OK) status = RD_SYNCHRONIZATION;
-    if (status == RD_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) status = RD_SYNCHRONIZATION;
+    if (status == RD_OK && rd::instantiate_graph(device, &exec, graph, main) != cudaSuccess) status = RD_SYNCHRONIZATION;
     cudaGetLastError();
   }
   const auto c1 = Clock::now();
@@ -176,7 +176,7 @@ extern "C" rd_status rd_develop_batch_graph(int device, rd_batch_item* items, in
       std::memcpy(stage + in_off[k], it.mosaic, sizeof(uint16_t) * it.row_stride * it.sensor.sensor_height);
     }
     const auto l0 = Clock::now();
-    if (cudaGraphLaunch(exec, main) != cudaSuccess || cudaStreamSynchronize(main) != cudaSuccess)
+    if (rd::launch_graph(device, exec, main) != cudaSuccess || cudaStreamSynchronize(main) != cudaSuccess)
       status = RD_SYNCHRONIZATION;
     if (launch_ms) *launch_ms = std::chrono::duration<double, std::milli>(Clock::now() - l0).count();
     for (int c = 0; c < chains && status == RD_OK; ++c) {

@@ -210,6 +210,10 @@ Status set_stream_priority(Context& ctx, bool high);
 // Gives kept blocks back until the context's footprint holds and no more than
 // `bytes` are kept.
 void trim_kept_blocks(Context& ctx, uint64_t bytes);
+// Instantiates a captured graph, or launches it, again after every context of the
+// device has given its kept blocks back where there was no memory for it.
+cudaError_t instantiate_graph(int device, cudaGraphExec_t* exec, cudaGraph_t graph, cudaStream_t stream);
+cudaError_t launch_graph(int device, cudaGraphExec_t exec, cudaStream_t stream);
 // Around a stream capture that the context's stream is to join: before it does,
 // and after the capture has ended.
 void begin_capture(Context& ctx);
