@@ -1043,7 +1043,6 @@ __device__ void estimate_site_warp(const OpposedParams& p, int x, int y, float* 
   const unsigned support = support_count ? support_mask(target, ch, p.levels) : 0u;
   if (support != 0) {
     const bool pair = __popc(support) == 2;
-    const int o0 = ch == 0 ? 1 : 0, o1 = ch == 2 ? 1 : 2;
     float ref = 0.0f, tratio = 0.0f;
     reference_value(target, support, ref);  // succeeds: the support's means are bright-clean
     const bool has_tratio = pair && log_ratio(target, support, tratio);
