@@ -76,19 +76,6 @@ RD_HD int length_symbol(int len, int* extra_bits, int* extra_value) {
   return 257 + 4 * e + 4 + group;
 }
 
-// Token that starts at position p of a run [a, b): positions a..b-1 each
-// repeat the byte before them (position a - 1 is a literal). Matches of
-// distance 1 cover the run greedily, 258 bytes at a time, and a tail shorter
-// than 3 bytes is sent as literals. Returns 0 when p lies inside a match,
-// 1 when p is a literal, or the length (3..258) of the match starting at p.
-RD_HD int run_token(int p, int a, int b) {
-  const int k = p - a;
-  const int q = k - k % MAX_RUN;
-  const int rest = b - a - q;
-  if (rest >= 3) return k == q ? (rest < MAX_RUN ? rest : MAX_RUN) : 0;
-  return 1;
-}
-
 RD_HD int clz64(uint64_t v) {
 #if defined(__CUDA_ARCH__)
   return __clzll((long long)v);
@@ -105,7 +92,7 @@ RD_HD int ctz64(uint64_t v) {
 }
 
 // A thread's share of a segment: CHUNK bytes at segment position c0, held in
-// 16 little-endian words (registers on the device when indexed by constants).
+// CHUNK_WORDS little-endian words (registers on the device when indexed by constants).
 constexpr int CHUNK = 32;  // below 64, so (1ull << count) - 1 is the mask of a full chunk
 constexpr int CHUNK_WORDS = CHUNK / 4;
 
@@ -154,8 +141,10 @@ RD_HD int ctz32(uint32_t v) {
 }
 
 // The chunk's tokens as bits: `literal` loses the bytes that matches cover,
-// `match` gets the first byte of each match that starts in the chunk
-// (run_token, a run at a time).
+// `match` gets the first byte of each match that starts in the chunk. A run is
+// the positions [a, b) that each repeat the byte before them. Matches of distance
+// 1 cover it greedily from a on, MAX_RUN bytes at a time; a rest of fewer than 3
+// is sent as literals.
 RD_HD void chunk_matches(uint64_t breaks, int c0, int count, int before, int after, uint32_t& literal,
                          uint32_t& match) {
   uint32_t rest = ~(uint32_t)breaks & (0xFFFFFFFFu >> (32 - count));
@@ -458,9 +447,9 @@ RD_HD uint32_t write_dynamic_header(BitWriter& w, bool final_block, const uint8_
 // Feeding a zero byte multiplies the register by x^8; with that, the CRC of a
 // concatenation A||B is (register after A) * x^(8|B|) xor (register of B from
 // zero), which lets each thread checksum its own bytes.
-RD_HD uint32_t gf2_times_x(uint32_t v) { return (v & 1u) ? (v >> 1) ^ CRC_POLY : v >> 1; }
+RD_HD constexpr uint32_t gf2_times_x(uint32_t v) { return (v & 1u) ? (v >> 1) ^ CRC_POLY : v >> 1; }
 
-RD_HD uint32_t gf2_mul(uint32_t a, uint32_t b) {
+RD_HD constexpr uint32_t gf2_mul(uint32_t a, uint32_t b) {
   uint32_t p = 0;
   for (int i = 0; i < 32; ++i) {
     if ((a >> (31 - i)) & 1u) p ^= b;
@@ -472,7 +461,8 @@ RD_HD uint32_t gf2_mul(uint32_t a, uint32_t b) {
 constexpr uint32_t GF2_ONE = 0x80000000u;  // x^0
 constexpr uint32_t GF2_X8 = 0x00800000u;   // x^8
 
-// xpow[k] = x^(8 * 2^k): the shift by 2^k zero bytes.
+// xpow[k] = x^(8 * 2^k): the shift by 2^k zero bytes, which the host harness
+// combines slices of any length with.
 struct CrcShifts {
   uint32_t xpow[40];
 };
@@ -499,6 +489,62 @@ RD_HD uint32_t crc_byte_entry(uint32_t byte) {
 
 RD_HD uint32_t crc_update(const uint32_t* table, uint32_t reg, const uint8_t* p, uint64_t n) {
   for (uint64_t i = 0; i < n; ++i) reg = table[(reg ^ p[i]) & 0xFFu] ^ (reg >> 8);
+  return reg;
+}
+
+// The register's four-byte step takes four tables: entry v of table k is byte v
+// followed by k zero bytes.
+RD_HD uint32_t crc_zero_bytes(const uint32_t* table0, uint32_t e, int k) {
+  for (int i = 0; i < k; ++i) e = (e >> 8) ^ table0[e & 255u];
+  return e;
+}
+
+// An encoded segment's chunk is checksummed by CRC_SHARES threads. Each takes
+// CRC_SHARE bytes, counted from the chunk's end, so that the registers of
+// neighbours combine over the same distances in every chunk: level j joins groups
+// of 2^j threads, the left one's register advanced over CRC_SHARE << j bytes.
+// Advancing is linear: one table entry per nibble. The share is an odd number of
+// words (the threads of a warp read different banks).
+constexpr uint32_t CRC_SHARE = 132;
+constexpr int CRC_LEVELS = 8, CRC_SHARES = 1 << CRC_LEVELS;
+static_assert(CRC_SHARE * CRC_SHARES >= SEG_CAP + 16, "the shares cover a chunk");
+struct CrcTree {
+  uint32_t t[CRC_LEVELS][8][16];
+};
+constexpr CrcTree crc_tree() {
+  CrcTree c{};
+  uint32_t step = GF2_ONE;
+  for (uint32_t k = 0; k < CRC_SHARE; ++k) step = gf2_mul(step, GF2_X8);
+  for (int j = 0; j < CRC_LEVELS; ++j) {
+    for (int n = 0; n < 8; ++n)
+      for (uint32_t v = 0; v < 16; ++v) c.t[j][n][v] = gf2_mul(v << (4 * n), step);
+    step = gf2_mul(step, step);
+  }
+  return c;
+}
+RD_HD uint32_t crc_advance(const uint32_t (&t)[8][16], uint32_t v) {
+  uint32_t r = 0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int n = 0; n < 8; ++n) r ^= t[n][(v >> (4 * n)) & 15u];
+  return r;
+}
+// The register of share `share` of `len` bytes: preset where the bytes begin,
+// zero before. byte(k) is byte k of them, word(k) bytes k .. k + 3.
+template <class Byte, class Word>
+RD_HD uint32_t crc_share(const uint32_t (&table)[4][256], int len, int share, Byte&& byte, Word&& word) {
+  const int end = len - (CRC_SHARES - 1 - share) * (int)CRC_SHARE, begin = end - (int)CRC_SHARE;
+  uint32_t reg = 0;
+  if (end > 0) {
+    int k = begin > 0 ? begin : 0;
+    if (begin <= 0) reg = 0xFFFFFFFFu;
+    for (; (end - k) & 3; ++k) reg = table[0][(reg ^ byte(k)) & 255u] ^ (reg >> 8);
+    for (; k < end; k += 4) {
+      reg ^= word(k);
+      reg = table[3][reg & 255u] ^ table[2][(reg >> 8) & 255u] ^ table[1][(reg >> 16) & 255u] ^ table[0][reg >> 24];
+    }
+  }
   return reg;
 }
 

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(FILTER_THREADS) png_filter_kernel(const void* 
 // any repeat as the test nearly every warp took both ways, and its CTA waited.
 // A literal chunk is taken word by word: with all 32 bytes extracted in advance,
 // and kept from the counting pass for the writing one, the packing spilled 280
-// bytes a thread, 1.2 GB of a 24 MP file, out to HBM (0.50 ms, histogram 0.21).
+// bytes a thread, 1.05 GB of a 24 MP file, out to HBM (0.50 ms, histogram 0.21).
 // 16-bit 24 MP: histogram 0.42 ms at first, 0.18 now, packing 0.90 and 0.38.
 constexpr int DEFLATE_THREADS = SEG / CHUNK;  // 1024
 constexpr int DEFLATE_WARPS = DEFLATE_THREADS / 32;
@@ -287,7 +287,7 @@ struct Chunk {
   uint64_t breaks;
 };
 
-// Bytes [c0, c0 + 64) of the segment that starts at `seg`, n bytes long. The
+// Bytes [c0, c0 + CHUNK) of the segment that starts at `seg`, n bytes long. The
 // stream buffer is padded to 16 bytes and segments start at multiples of SEG,
 // so whole 16-byte loads stay inside it; bytes past n are masked by count.
 __device__ __forceinline__ void load_chunk(const uint8_t* __restrict__ seg, int n, Chunk& ch) {
@@ -738,44 +738,8 @@ struct ChunkParams {
   uint32_t nseg;
 };
 
-// Each thread takes CRC_SHARE bytes of a chunk, counted from its end, so that
-// the registers of neighbours combine over the same distances in every chunk:
-// level j joins groups of 2^j threads, the left one's register advanced over
-// CRC_SHARE << j bytes. Advancing is linear: one table entry per nibble. The
-// share is an odd number of words (the threads of a warp read different banks).
-constexpr uint32_t CRC_SHARE = 132;
-constexpr int CRC_LEVELS = 8;
-static_assert(CRC_SHARE * CHUNK_THREADS >= SEG_CAP + 16 && CHUNK_THREADS == 1 << CRC_LEVELS, "the shares cover a chunk");
-struct CrcTree {
-  uint32_t t[CRC_LEVELS][8][16];
-};
-constexpr uint32_t crc_times(uint32_t a, uint32_t b) {  // gf2_mul
-  uint32_t r = 0;
-  for (int i = 0; i < 32; ++i) {
-    if (a & 0x80000000u) r ^= b;
-    a <<= 1;
-    b = (b >> 1) ^ ((b & 1u) ? CRC_POLY : 0u);
-  }
-  return r;
-}
-constexpr CrcTree crc_tree() {
-  CrcTree c{};
-  uint32_t step = GF2_ONE;
-  for (uint32_t k = 0; k < CRC_SHARE; ++k) step = crc_times(step, GF2_X8);
-  for (int j = 0; j < CRC_LEVELS; ++j) {
-    for (int n = 0; n < 8; ++n)
-      for (uint32_t v = 0; v < 16; ++v) c.t[j][n][v] = crc_times(v << (4 * n), step);
-    step = crc_times(step, step);
-  }
-  return c;
-}
+static_assert(CHUNK_THREADS == CRC_SHARES, "a thread per share");
 __device__ const CrcTree CRC_TREE = crc_tree();
-__device__ __forceinline__ uint32_t crc_advance(const uint32_t (&t)[8][16], uint32_t v) {
-  uint32_t r = 0;
-#pragma unroll
-  for (int n = 0; n < 8; ++n) r ^= t[n][(v >> (4 * n)) & 15u];
-  return r;
-}
 
 // The segment's block lies in shared memory from byte 16 on, the chunk's length
 // and type (and the zlib header) in front of it. CRC-32 takes four bytes a step
@@ -801,11 +765,7 @@ __global__ void __launch_bounds__(CHUNK_THREADS) png_chunk_kernel(const __grid_c
   for (uint32_t v = tid; v < (nb + 15) / 16; v += CHUNK_THREADS) reinterpret_cast<uint4*>(buf + DATA)[v] = __ldg(src + v);
   __syncthreads();
 #pragma unroll
-  for (int k = 1; k < 4; ++k) {
-    uint32_t e = table[0][tid];
-    for (int i = 0; i < k; ++i) e = (e >> 8) ^ table[0][e & 255u];
-    table[k][tid] = e;
-  }
+  for (int k = 1; k < 4; ++k) table[k][tid] = crc_zero_bytes(table[0], table[0][tid], k);
   if (tid == 0) {
     uint8_t* c = buf + start;
     for (int k = 0; k < 4; ++k) c[k] = (uint8_t)(dl >> (24 - 8 * k));
@@ -827,18 +787,9 @@ __global__ void __launch_bounds__(CHUNK_THREADS) png_chunk_kernel(const __grid_c
   const uint32_t* words = reinterpret_cast<const uint32_t*>(buf);
   auto word_at = [&](uint32_t o) { return __funnelshift_r(words[o >> 2], words[(o >> 2) + 1], 8 * (o & 3u)); };
   // CRC-32 over the chunk type and data, each thread over its own bytes.
-  const int crc_len = (int)(4 + dl), b1 = crc_len - (CHUNK_THREADS - 1 - tid) * (int)CRC_SHARE, b0 = b1 - (int)CRC_SHARE;
-  uint32_t reg = 0;
-  if (b1 > 0) {
-    const uint32_t o = start + 4;
-    int k = max(b0, 0);
-    if (b0 <= 0) reg = 0xFFFFFFFFu;
-    for (; (b1 - k) & 3; ++k) reg = table[0][(reg ^ buf[o + k]) & 255u] ^ (reg >> 8);
-    for (; k < b1; k += 4) {
-      reg ^= word_at(o + k);
-      reg = table[3][reg & 255u] ^ table[2][(reg >> 8) & 255u] ^ table[1][(reg >> 16) & 255u] ^ table[0][reg >> 24];
-    }
-  }
+  const uint32_t from = start + 4;
+  uint32_t reg = crc_share(table, (int)(4 + dl), tid, [&](int k) { return (uint32_t)buf[from + k]; },
+                           [&](int k) { return word_at(from + k); });
   // Groups to the left of the chunk's start have a zero register.
 #pragma unroll
   for (int j = 0; j < 5; ++j) reg = crc_advance(tree.t[j], __shfl_up_sync(FULL_MASK, reg, 1 << j)) ^ reg;
